@@ -252,7 +252,7 @@ struct PhaseArgs {
   int *M, *Mt, *CS;         // the tile behind `v`, written by the apply pass
   const int32_t* hubs;      // hub vertex ids, ascending
   const int32_t* batch_hub; // first hub of each batch (batches + 1 entries)
-  const int2* units;        // per batch: vertex pairs of degree <= 64, or (v, -2) for 64 < degree <= 128
+  const int2* units;        // per batch: vertex pairs of degree <= 64, or (v, -2) for a single one
   const int32_t* unit_ptr;  // first unit of each batch (batches + 1 entries)
   const int64_t* chunk_ptr;
   int n, bs, maxitr, W;
@@ -301,6 +301,7 @@ void launch_merge_relabel(int n, int B, int32_t* part, const int32_t* root, int3
 void nodal_configure(int device);
 // grid of the persistent nodal kernel on `device` (0: not available)
 int nodal_phase_grid(int device);
+int nodal_phase_warps();   // warps of one of its CTAs
 int nodal_gang_grid(int device);
 // largest B whose hub tables fit the persistent kernel's shared memory
 int nodal_phase_max_blocks();

@@ -687,7 +687,11 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
                        double model_d, int32_t maxitr, int stats, int grid, bool timed) {
   const int32_t n = hg_->n;
   const int32_t nb = (n + bs_ - 1) / bs_;
-  if (batch_hub_bs_ != bs_) {   // first hub of each batch, for this batch size
+  // a vertex per warp while a batch has no more vertices than the grid has
+  // warps (one wave either way, and a lone vertex is through sooner); two a
+  // warp beyond that, and in the gang, whose jobs share the grid
+  const bool single = !gang_ && bs_ <= static_cast<int64_t>(grid) * nodal_phase_warps();
+  if (batch_hub_bs_ != bs_ || units_single_ != single) {   // first hub of each batch, for this batch size
     const std::vector<int32_t>& hub_ids = gr_->hub_ids;
     std::vector<int32_t> bh(static_cast<size_t>(nb) + 1);
     for (int32_t b = 0; b <= nb; b++) {
@@ -707,7 +711,7 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
       for (int32_t v = beg; v < end; v++) {
         const int64_t deg = (hg_->out_ptr[v + 1] - hg_->out_ptr[v]) + (hg_->in_ptr[v + 1] - hg_->in_ptr[v]);
         if (deg > kHubDegree) continue;
-        if (deg > kHubDegree / 2) {
+        if (single || deg > kHubDegree / 2) {
           mid.push_back(v);
         } else if (pending < 0) {
           pending = v;
@@ -748,6 +752,7 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
       USAP_CUDA(cudaMemcpyAsync(ud, un.data(), sizeof(int32_t) * un.size(), cudaMemcpyHostToDevice, st_));
     wait();
     batch_hub_bs_ = bs_;
+    units_single_ = single;
   }
   PhaseArgs pa;
   pa.a = nodal_args(part, B, 0, 0, stage, seed, stats);

@@ -324,6 +324,7 @@ class Job {
   int32_t* unit_ptr_ = nullptr;      // first work unit of each batch
   int2* units_ = nullptr;            // work units of the persistent kernel
   int32_t batch_hub_bs_ = 0;
+  bool units_single_ = false;        // units_ holds one vertex per unit
   int32_t batch_hub_cap_ = 0;
   int32_t *dout_ = nullptr, *din_ = nullptr;
   int *M_ = nullptr, *Mt_ = nullptr, *CS_ = nullptr;
