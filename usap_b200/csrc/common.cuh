@@ -215,6 +215,7 @@ static __device__ const double2 kRefLogTab[] = {
 #include "ref_log_table.inc"
 };
 constexpr int kRefLogK0 = 38;   // table index of k = 0
+constexpr int kRefLogSize = sizeof(kRefLogTab) / sizeof(kRefLogTab[0]);
 
 __device__ __forceinline__ float ref_logf(float x) {
   if (!(x > 0.0f)) return x == 0.0f ? __int_as_float(0xff800000) : __int_as_float(0x7fc00000);
@@ -257,24 +258,52 @@ __device__ __forceinline__ float ref_logf(float x) {
   return __double2float_rn(__dadd_rn(hi, l1p));
 }
 
-// ref_logf for x > 0 (+inf included) without branches: the same operations
-// on the same values, the special cases chosen by selects, so that several
-// evaluations can be interleaved by the compiler.
-__device__ __forceinline__ float ref_logf_pos(float x) {
+// x / p rounded to nearest for positive normal x and p whose quotient and
+// residuals stay in the normal range, without the branch of an operator's
+// special cases (so that several evaluations interleave): Markstein's
+// method -- a Newton step on the approximate reciprocal, then two residual
+// corrections of the quotient, each a fused multiply-add.  Equal to
+// __fdiv_rn for every pair of 24-bit mantissas (compared for all 2^46).
+// Other inputs give some value.
+__device__ __forceinline__ float quot_rn(float x, float p) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(p));
+  y = __fmaf_rn(y, __fmaf_rn(-p, y, 1.0f), y);
+  float q = __fmul_rn(x, y);
+  q = __fmaf_rn(__fmaf_rn(-p, q, x), y, q);
+  return __fmaf_rn(__fmaf_rn(-p, q, x), y, q);
+}
+
+// kRefLogTab in shared memory, for kernels that evaluate many terms: the
+// lanes' entries differ, and the little L1 that a large shared-memory
+// allocation leaves does not hold the table against streaming loads.
+// ref_tab_fill: CTA-collective, before the first use (and a __syncthreads).
+__device__ __forceinline__ double2* ref_tab() {
+  __shared__ double2 tab[kRefLogSize];
+  return tab;
+}
+__device__ __forceinline__ void ref_tab_fill() {
+  for (int i = threadIdx.x; i < kRefLogSize; i += blockDim.x) ref_tab()[i] = kRefLogTab[i];
+}
+
+// ref_logf of a quotient x / prod with 1 <= x, prod < 2^48 (a normal, finite,
+// positive float), without branches: the same operations on the same values
+// as ref_logf, so that several evaluations interleave.  Any other input
+// gives a value that the caller discards (the table index is in range for
+// every bit pattern).
+__device__ __forceinline__ float ref_logf_quot(float x) {
   const unsigned u = __float_as_uint(x);
-  int e = static_cast<int>(u >> 23);
-  unsigned frac = u & 0x7fffffu;
-  const bool sub = e == 0;   // subnormal: shift the leading one into the hidden bit
-  const int sh = sub ? __clz(static_cast<int>(frac)) - 8 : 0;
-  frac = (frac << sh) & 0x7fffffu;
-  e = (sub ? 1 - sh : e) - 127;
-  const bool half = frac >= 0x3504F4u;
-  e += half ? 1 : 0;
-  const unsigned long long mbits = ((half ? 1022ull : 1023ull) << 52) | (static_cast<unsigned long long>(frac) << 29);
-  const int k = half ? static_cast<int>((frac + 0x10000u) >> 17) - 64 : static_cast<int>((frac + 0x8000u) >> 16);
-  const double m = __longlong_as_double(static_cast<long long>(mbits));
-  const double2 t = __ldg(kRefLogTab + kRefLogK0 + (u >= 0x7f800000u ? 0 : k));
-  const double w = __dsub_rn(__dmul_rn(m, t.x), 1.0);
+  // e = exponent of x, one more where the fraction is at least sqrt(2)'s
+  // (0x3504F4); d = (m - 1) 2^23 with m = x / 2^e, negative when m < 1
+  const int e = static_cast<int>(u - 0x3f3504f4u) >> 23;
+  const unsigned mb = u - (static_cast<unsigned>(e) << 23);
+  const int d = static_cast<int>(mb - 0x3f800000u);
+  // k = 128 (m - 1) rounded half up: d / 2^16, or d / 2^17 below one, where
+  // a unit of d is half as large
+  const int k = ((d >> (15 - (d >> 31))) + 1) >> 1;
+  const double m = __hiloint2double(static_cast<int>((mb >> 3) + (896u << 20)), static_cast<int>(mb << 29));
+  const double2 t = ref_tab()[kRefLogK0 + k];
+  const double w = __fma_rn(m, t.x, -1.0);   // exact, as m * t.x is
   double q = -1.0 / 8.0;
   q = __fma_rn(q, w, 1.0 / 7.0);
   q = __fma_rn(q, w, -1.0 / 6.0);
@@ -283,16 +312,20 @@ __device__ __forceinline__ float ref_logf_pos(float x) {
   q = __fma_rn(q, w, 1.0 / 3.0);
   q = __fma_rn(q, w, -1.0 / 2.0);
   const double l1p = __fma_rn(__dmul_rn(w, w), q, w);
-  const double ed = __dsub_rn(__longlong_as_double(0x4338000000000000ll + e), 6755399441055744.0);
+  // e as a double: 2^52 + 2^51 + 2^31 + e, minus the offset
+  const double ed = __dsub_rn(__hiloint2double(0x43380000, static_cast<int>(static_cast<unsigned>(e) ^ 0x80000000u)),
+                              6755399441055744.0 + 2147483648.0);
   const double hi = __fma_rn(ed, 0.69314718055994530942, t.y);
-  const float r = __double2float_rn(__dadd_rn(hi, l1p));
-  return u >= 0x7f800000u ? x : r;   // +inf
+  return __double2float_rn(__dadd_rn(hi, l1p));
 }
 
-// ref_term(x, prod) where x != 0, else 0, without branches (x, prod >= 0)
-__device__ __forceinline__ float ref_term_nz(int x, long long prod) {
-  const float xf = __int2float_rn(x ? x : 1);
-  const float t = __fmul_rn(xf, ref_logf_pos(__fdiv_rn(xf, __ll2float_rn(x ? prod : 1))));
+// ref_term(x, da * db) where x != 0, else 0, without branches (x >= 0).  The
+// degrees come as floats: they are below 2^24, so exact, and the float
+// product of two of them is the reference's long product rounded to float.
+// Where x > 0 neither degree is zero: both count x among their edges.
+__device__ __forceinline__ float ref_term_nz(int x, float da, float db) {
+  const float xf = __int2float_rn(x);
+  const float t = __fmul_rn(xf, ref_logf_quot(quot_rn(xf, __fmul_rn(da, db))));
   return x ? t : 0.0f;
 }
 

@@ -66,11 +66,12 @@ LaunchCount& launch_count();
 // Vertices whose degree exceeds kHubDegree are proposed by a whole CTA;
 // its neighbour-block hash holds up to kHubSmemSlots entries in shared
 // memory (3 ints per slot), larger ones use the vertex's global region.
-constexpr int kHubDegree = 128;
+constexpr int kHubDegree = 192;
+constexpr int kPairDegree = 64;   // two vertices up to this degree share a warp (a half-warp each)
 constexpr int kHubSmemSlots = 16384;
 // the persistent kernels' hub table (shared memory): hubs whose table is
 // larger get a region of global memory, so those kernels take any B
-constexpr int kPhaseHubSlots = 8192;
+constexpr int kPhaseHubSlots = 4096;
 
 // process-wide device memory pool and host tables (devmem.cu)
 void pool_configure(int device);
@@ -178,6 +179,7 @@ struct GraphDev {
   int64_t e = 0;
   int64_t wtot = 0;
   bool unit = true;
+  int32_t maxdeg = 0, maxk = 0;   // most neighbours of a vertex, largest weighted degree
   int32_t *src = nullptr, *dst = nullptr, *w = nullptr;
   int32_t *out_ptr = nullptr, *out_idx = nullptr, *out_w = nullptr;
   int32_t *in_ptr = nullptr, *in_idx = nullptr, *in_w = nullptr;
@@ -225,6 +227,9 @@ struct NodalArgs {
   float* Trow;            // M[b,i] log(M[b,i] / (d_in[i] d_out[b]))
   float* Tcol;            // M[i,b] log(M[i,b] / (d_out[i] d_in[b]))
   int tld;
+  int sparse;             // precision mode 3: skip the tile's empty cells (float_ds_sparse)
+  int coop;               // precision mode 3, persistent kernels: a CTA evaluates its float dS together
+  int hub_units;          // ... and a warp proposes for any vertex (no hub CTAs)
 };
 
 struct MergeArgs {
@@ -252,7 +257,7 @@ struct PhaseArgs {
   int *M, *Mt, *CS;         // the tile behind `v`, written by the apply pass
   const int32_t* hubs;      // hub vertex ids, ascending
   const int32_t* batch_hub; // first hub of each batch (batches + 1 entries)
-  const int2* units;        // per batch: vertex pairs of degree <= 64, or (v, -2) for a single one
+  const int2* units;        // per batch: vertex pairs of degree <= 64, or (v, -2) for one vertex (64 < degree <= 192, or any)
   const int32_t* unit_ptr;  // first unit of each batch (batches + 1 entries)
   const int64_t* chunk_ptr;
   int n, bs, maxitr, W;
@@ -301,6 +306,9 @@ void launch_merge_relabel(int n, int B, int32_t* part, const int32_t* root, int3
 void nodal_configure(int device);
 // grid of the persistent nodal kernel on `device` (0: not available)
 int nodal_phase_grid(int device);
+// precision mode 3: whether the float dS packs the non-zero cells of its rows
+// before it evaluates terms (a tile of B x B cells, `e` edges)
+bool float_ds_sparse(int64_t e, int32_t B, bool coop);
 int nodal_phase_warps();   // warps of one of its CTAs
 int nodal_gang_grid(int device);
 // largest B whose hub tables fit the persistent kernel's shared memory

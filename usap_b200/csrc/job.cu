@@ -279,8 +279,11 @@ std::shared_ptr<GraphResident> load_graph(int device, const usap_graph& in, Host
   std::vector<int64_t> hi_off(n, -1);
   std::vector<int32_t> hubs;
   int64_t hi_slots = 0;
+  int32_t maxdeg = 0, maxk = 0;
   for (int32_t v = 0; v < n; v++) {
     int deg = (h.out_ptr[v + 1] - h.out_ptr[v]) + (h.in_ptr[v + 1] - h.in_ptr[v]);
+    maxdeg = std::max(maxdeg, deg);
+    maxk = std::max(maxk, std::max(h.kout[v], h.kin[v]));
     if (deg > kHubDegree) {
       hubs.push_back(v);
       int cap = 1 << hash_lg(deg);
@@ -310,6 +313,8 @@ std::shared_ptr<GraphResident> load_graph(int device, const usap_graph& in, Host
   g.n = n;
   g.e = h.e;
   g.wtot = wtot;
+  g.maxdeg = maxdeg;
+  g.maxk = maxk;
   g.unit = h.unit;
   long long up_bytes = 0;
   auto up = [&](int32_t** d, const std::vector<int32_t>& v) {
@@ -485,8 +490,8 @@ void Job::ensure_capacity(int32_t B, int32_t K, int32_t dense_max, int32_t maxit
     dfree(dout_); dfree(din_); dfree(best_s_); dfree(best_q_); dfree(best_x_);
     dfree(skeys_); dfree(skeys_alt_); dfree(sidx_); dfree(sidx_alt_);
     dfree(union_work_); dfree(root_); dfree(present_); dfree(newlabel_); dfree(merged_dev_);
-    dalloc(&dout_, B);
-    dalloc(&din_, B);
+    dalloc(&dout_, B + 1);   // readable in pairs
+    dalloc(&din_, B + 1);
     dalloc(&best_s_, B);
     dalloc(&best_q_, B);
     dalloc(&best_x_, B);
@@ -646,6 +651,9 @@ NodalArgs Job::nodal_args(int32_t* part, int32_t B, int32_t beg, int32_t end, ui
   a.Trow = nullptr;
   a.Tcol = nullptr;
   a.tld = 0;
+  a.sparse = prec_ == 3 && float_ds_sparse(g_.e, B, false) ? 1 : 0;
+  a.coop = 0;
+  a.hub_units = 0;
   if (stats == 2) {   // replay: per-vertex proposals
     a.prop_s = rp_s_;
     a.prop_q = rp_q_;
@@ -687,9 +695,7 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
                        double model_d, int32_t maxitr, int stats, int grid, bool timed) {
   const int32_t n = hg_->n;
   const int32_t nb = (n + bs_ - 1) / bs_;
-  // a vertex per warp while a batch has no more vertices than the grid has
-  // warps (one wave either way, and a lone vertex is through sooner); two a
-  // warp beyond that, and in the gang, whose jobs share the grid
+  // a vertex per warp while a batch fits the grid's warps that way, else two
   const bool single = !gang_ && bs_ <= static_cast<int64_t>(grid) * nodal_phase_warps();
   if (batch_hub_bs_ != bs_ || units_single_ != single) {   // first hub of each batch, for this batch size
     const std::vector<int32_t>& hub_ids = gr_->hub_ids;
@@ -699,7 +705,7 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
       bh[b] = static_cast<int32_t>(std::lower_bound(hub_ids.begin(), hub_ids.end(), v) - hub_ids.begin());
     }
     // work units: pairs of vertices of degree <= 64 (half-warps), single
-    // vertices of degree <= 128 (warps); hubs are proposed by whole CTAs
+    // vertices of degree <= 192 (warps); hubs are proposed by whole CTAs
     std::vector<int32_t> up(static_cast<size_t>(nb) + 1, 0);
     std::vector<int32_t> un;
     un.reserve(2 * static_cast<size_t>(n));
@@ -711,7 +717,7 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
       for (int32_t v = beg; v < end; v++) {
         const int64_t deg = (hg_->out_ptr[v + 1] - hg_->out_ptr[v]) + (hg_->in_ptr[v + 1] - hg_->in_ptr[v]);
         if (deg > kHubDegree) continue;
-        if (single || deg > kHubDegree / 2) {
+        if (single || deg > kPairDegree) {
           mid.push_back(v);
         } else if (pending < 0) {
           pending = v;
@@ -781,10 +787,17 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
   pa.bar_hold = bar_test_hold_;
   bar_test_hold_ = -1;   // one launch only
   bar_test_timeout_ns_ = 0;
+  if (prec_ == 3) {
+    pa.a.coop = 1;
+    pa.a.sparse = float_ds_sparse(g_.e, B, true) ? 1 : 0;
+    // a warp's table counts 16 bits a block and direction; beyond 2048
+    // neighbours a CTA is faster than a warp
+    pa.a.hub_units = !pa.a.shadow && B <= 768 && g_.maxk < 65536 && g_.maxdeg <= 2048;
+  }
   // precision mode 3: the old-state term tables of the persistent kernels,
-  // single-job and gang (B <= kRefTabMaxB; above it the per-cell tables
-  // cost more than the proposals' own evaluation)
-  if (prec_ == 3 && B <= kRefTabMaxB) {
+  // single-job and gang (one pass over the tile and a grid barrier per
+  // batch), where the proposals' own evaluation costs more: see kRefTabMin
+  if (pa.a.coop && !pa.a.sparse && (gang_ || static_cast<int64_t>(bs_) * B > kRefTabMin * grid)) {
     const size_t cells = static_cast<size_t>(ld_) * ld_;
     if (cells > tcap_) {
       dfree(Trow_);

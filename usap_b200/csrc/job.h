@@ -329,7 +329,11 @@ class Job {
   int32_t *dout_ = nullptr, *din_ = nullptr;
   int *M_ = nullptr, *Mt_ = nullptr, *CS_ = nullptr;
   // precision mode 3: old-state term tables of the persistent kernel (ld_ x ld_ floats each)
-  static constexpr int32_t kRefTabMaxB = 4096;
+  // where proposals per CTA x B exceeds kRefTabMin: below it the pass over the
+  // tile and its grid barrier (3 us) cost more than they save (batches with
+  // and without the tables: N = 50000, B = 96, 3250: 37.4 and 39.0 us; N =
+  // 20000, B = 154, 2080: 33.3 and 33.1 us; B = 39: 22.1 and 20.4 us)
+  static constexpr int64_t kRefTabMin = 3200;
   float *Trow_ = nullptr, *Tcol_ = nullptr;
   size_t tcap_ = 0;
   int ld_ = 0, cld_ = 0;

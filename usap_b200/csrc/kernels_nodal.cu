@@ -7,7 +7,8 @@
 // the buffered moves, rebuilds M from scratch and tests convergence.
 //
 // Here one warp proposes for one vertex (one CTA for vertices of degree
-// above kHubDegree, so a hub does not set the batch's tail).  The target is
+// above kHubDegree, so a hub does not set the batch's tail; up to that, and
+// in precision 3 mostly beyond, a warp is faster).  The target is
 // drawn in block-id order: on the dense tile through per-row chunk sums of
 // M[u,:]+M[:,u] (chunks of 128 blocks, kept current by the same delta
 // updates as M), on the sparse views by binary search of cumulative counts.
@@ -32,7 +33,9 @@
 // start, proposals and apply; it removes the launch gaps that otherwise
 // cost about half of each batch.  There each CTA applies the moves it
 // accepted itself (listed in shared memory while proposing), and for small
-// B the proposals read a per-batch copy of the tile in shared memory.
+// B the proposals read a per-batch copy of the tile in shared memory.  In
+// precision 3 a wave's proposals are only drawn by their warps; the CTA then
+// evaluates their float dS together.
 // State written inside that kernel (the partition, M, degrees, chunk sums,
 // moves) is otherwise read through L2 (ld.cg); the non-coherent path is
 // used only for data that no phase writes.  The gang kernel runs the same
@@ -468,61 +471,127 @@ __device__ __forceinline__ long long finalize_grp(const NodalArgs& a, const Grp<
 
 // Precision mode 3: the reference's single-precision dS of v (block r)
 // moving to s, _propose_new_partition_nodal (graph_parallel.hpp:1066-1215),
-// in its float arithmetic and term order, by a group of G lanes:
+// in its float arithmetic and term order:
 //  1. the old terms of rows r, s and (i not in {r, s}) columns r, s, block
 //     by block (:1096-1114);
 //  2. the four new 2x2 terms, the row entries adjusted by v's out-edges only
 //     (:1180-1195; the in-edge adjustment is commented out at :1135-1142);
 //  3. the new terms of rows and columns for i not in {r, s} (:1196-1215),
 //     the entries adjusted by v's out-weight (rows) and in-weight (columns)
-//     towards block i, looked up in the group's neighbour-block table.
-// A round covers G blocks: lane l loads the entries of block base + l of
-// the four rows (the next round's loads are issued before this round's
-// terms are evaluated).  The lanes evaluate the terms of their block, and
-// the terms are then added to one float accumulator in
-// the reference's order -- lane after lane, and within a lane in the
-// reference's term order (float addition does not reassociate), through the
-// group's shared-memory buffer `buf` (ref32_accumulate).  Rounds whose four
-// rows are empty in every lane are skipped.  Every lane returns the same
-// value.  Rr, Rs,
-// Sr, Ss: M[r,r], M[r,s], M[s,r], M[s,s]; wor, wos: v's out-weight to
-// blocks r and s.
-// One round of the chain: lane l's four terms (0 where the reference skips
-// a zero count) are staged in buf[4 l .. 4 l + 3] (buf: 4 G floats of the
-// group's shared memory, 16-byte aligned), and every lane then adds (or
-// subtracts) all 4 G of them to its copy of the accumulator in that order.
-// Adding a zero term leaves the float sum unchanged: the accumulator starts
-// at +0 and round-to-nearest never makes it -0, so x + 0 = x holds for every
-// value it takes (infinities and NaN included).  The loop has the same trip
-// count in every group, so the two half-warp groups of a warp run it in
-// step, one shared-memory broadcast load per four terms.
+//     towards block i, from the vertex's neighbour-block weights.
+// The terms can be evaluated in any order, but float addition does not
+// reassociate, so they are added one after the other, in the reference's
+// order, to one accumulator.  The persistent kernels evaluate the terms of
+// all of a CTA's proposals together and give every chain a thread
+// (coop_eval, coop_eval_sparse); ref32_eval is the form of a single warp,
+// for the per-batch kernels.  Adding a zero term (an empty cell) leaves the
+// float sum unchanged: the accumulator starts at +0 and round-to-nearest
+// never makes it -0, so x + 0 = x holds for every value it takes (infinities
+// and NaN included).
+//
+// One round of a warp's chain: lane l's four terms (block base + l) are
+// staged in buf[4 l .. 4 l + 3] (buf: 4 G floats of shared memory, 16-byte
+// aligned), and every lane then adds (or subtracts) all 4 G of them to its
+// copy of the accumulator in that order.
 template <int G>
-__device__ __forceinline__ float ref32_accumulate(const Grp<G>& g, float dS, float t0, float t1, float t2,
-                                                  float t3, bool sub, float* buf) {
-  reinterpret_cast<float4*>(buf)[g.gl] = make_float4(t0, t1, t2, t3);
-  g.sync();
+__device__ __forceinline__ float ref32_accumulate(float dS, int gl, float t0, float t1, float t2, float t3, bool sub,
+                                                  float* buf) {
+  reinterpret_cast<float4*>(buf)[gl] = make_float4(t0, t1, t2, t3);
+  __syncwarp();
 #pragma unroll 8
   for (int j = 0; j < G; j++) {
     const float4 q = reinterpret_cast<const float4*>(buf)[j];
     if (sub) dS = __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(dS, q.x), q.y), q.z), q.w);
     else dS = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(dS, q.x), q.y), q.z), q.w);
   }
-  g.sync();   // the next round overwrites buf
+  __syncwarp();   // the next round overwrites buf
   return dS;
 }
 
+// How a group keeps its vertex's out- and in-weight towards each block:
+// hashed by block (key, then out-, then in-weights), or in an array over all
+// blocks, whose update is one addition and whose lookup one load
+constexpr int kNbrHash = 0;
+constexpr int kNbr8 = 1;    // 2 bytes a block: out, in (unit weights, degree <= 255)
+constexpr int kNbr16 = 2;   // 4 bytes a block: out, in
+
+// A proposal: v moves from block r to s.  In precision 3 it lies in shared
+// memory until its float dS is evaluated.
+struct __align__(16) Pend {
+  int mode, job;   // kNbr*; the gang's job
+  bool hub;        // its chunks are not listed
+  const int* tab;  // v's neighbour-block weights (kNbr8, kNbr16), or the hash's keys
+  const int *two, *twi;   // the hash's out- and in-weights
+  float4 fo, fn;   // degree factors of rows r, s and columns r, s, old and new state
+  int v, r, s, deg, scanned, noccupied;
+  int dr_out, dr_in, ds_out, ds_in, kout, kin;
+  int Rr, Rs, Sr, Ss, wor, wos;
+  int cap, lg;     // the group's neighbour-block table
+  long long acc;   // the exact value beside it (shadow)
+  int ninf;
+};
+
+// the proposals of a CTA that are evaluated together
+constexpr int kMaxPend = 48;   // two per warp and wave
+constexpr int kSlot = 256;     // floats of a slot of coop_eval_sparse: 64 blocks x 4 rows
+constexpr int kMaxSlots = 48;
+struct PendList {
+  Pend p[kMaxPend];
+  int n;
+};
+
+// v's out- and in-weight towards block i
+__device__ __forceinline__ void nbr_weights(const Pend& q, int i, int* wo, int* wi) {
+  if (q.mode == kNbr8) {
+    const unsigned w = reinterpret_cast<const unsigned short*>(q.tab)[i];
+    *wo = w & 0xff;
+    *wi = w >> 8;
+  } else if (q.mode == kNbr16) {
+    const unsigned w = q.tab[i];
+    *wo = w & 0xffff;
+    *wi = w >> 16;
+  } else {
+    unsigned h = hash_slot(i, q.lg);
+    int k;
+    while ((k = q.tab[h]) != i && k != -1) h = (h + 1) & (q.cap - 1);   // (a free slot holds no weights)
+    *wo = q.two[h];
+    *wi = q.twi[h];
+  }
+}
+
+__device__ __forceinline__ void set_factors(Pend& q) {
+  q.fo = make_float4(q.dr_out, q.ds_out, q.dr_in, q.ds_in);
+  q.fn = make_float4(q.dr_out - q.kout, q.ds_out + q.kout, q.dr_in - q.kin, q.ds_in + q.kin);
+}
+
+// the four new 2x2 terms (subtracted, in this order)
+__device__ __forceinline__ void corner_terms(const Pend& q, float* c0, float* c1, float* c2, float* c3) {
+  const int dor_n = q.dr_out - q.kout, dos_n = q.ds_out + q.kout;
+  const int dir_n = q.dr_in - q.kin, dis_n = q.ds_in + q.kin;
+  const int rr_r = q.Rr - q.wor, rr_s = q.Rs - q.wos, sr_r = q.Sr + q.wor, sr_s = q.Ss + q.wos;
+  *c0 = rr_r ? ref_term(rr_r, static_cast<long long>(dir_n) * dor_n) : 0.0f;
+  *c1 = rr_s ? ref_term(rr_s, static_cast<long long>(dis_n) * dor_n) : 0.0f;
+  *c2 = sr_r ? ref_term(sr_r, static_cast<long long>(dir_n) * dos_n) : 0.0f;
+  *c3 = sr_s ? ref_term(sr_s, static_cast<long long>(dis_n) * dos_n) : 0.0f;
+}
+
+__device__ __forceinline__ float ref32_corner(float dS, const Pend& q) {
+  float c0, c1, c2, c3;
+  corner_terms(q, &c0, &c1, &c2, &c3);
+  return __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(dS, c0), c1), c2), c3);
+}
+
 // (not inlined: it runs after the group's other work is done, and a call
-// gives it the registers the proposal code held)
+// gives it the registers the proposal code held.)
 template <class Ops, int G>
 __device__ __noinline__ float ref32_nodal(const Ops ops, const int32_t* __restrict__ din_p,
                                           const int32_t* __restrict__ dout_p, const float* Trow,
-                                          const float* Tcol, int tld, int r, int s, int dr_out, int dr_in,
-                                          int ds_out, int ds_in, int kout, int kin, int Rr, int Rs, int Sr, int Ss,
-                                          int wor, int wos, const int* key, const int* two, const int* twi, int cap,
-                                          int lg, float* buf) {
+                                          const float* Tcol, int tld, const Pend& q, const int* key, const int* two,
+                                          const int* twi, float* buf) {
   using LDT = typename Ops::LdT;
   const Grp<G> g(static_cast<int>(threadIdx.x & 31));
-  const int B = ops.B;
+  const int B = ops.B, r = q.r, s = q.s;
+  const int cap = q.cap, lg = q.lg;
   float dS = 0.0f;
   // Every round first issues the loads of the next round (pure reads of the
   // batch-start state), so that their L2 latency overlaps this round's
@@ -545,13 +614,14 @@ __device__ __noinline__ float ref32_nodal(const Ops ops, const int32_t* __restri
     for (int base = 0; base < B; base += G) {
       const float t0 = n0, t1 = n1, t2 = n2, t3 = n3;
       tload(base + G + g.gl);
-      dS = ref32_accumulate<G>(g, dS, t0, t1, t2, t3, false, buf);
+      dS = ref32_accumulate<G>(dS, g.gl, t0, t1, t2, t3, false, buf);
     }
   }
   // a round's entries of rows r, s (R, S), columns r, s (Rc, Sc) and the
   // degrees of its block (d_in: di, d_out: dn)
   int nR, nS, nRc, nSc, ndi, ndn;
   if (!Trow) {
+    const float dor = q.fo.x, dos = q.fo.y, dir = q.fo.z, dis = q.fo.w;
     auto oload = [&](int i) {
       nR = nS = nRc = nSc = ndi = ndn = 0;
       if (i < B) {
@@ -567,23 +637,19 @@ __device__ __noinline__ float ref32_nodal(const Ops ops, const int32_t* __restri
     };
     oload(g.gl);
     for (int base = 0; base < B; base += G) {
-      const int R = nR, S = nS, Rc = nRc, Sc = nSc, di = ndi, dn = ndn;
+      const int R = nR, S = nS, Rc = nRc, Sc = nSc;
+      const float di = __int2float_rn(ndi), dn = __int2float_rn(ndn);
       oload(base + G + g.gl);
-      if (!g.any((R | S | Rc | Sc) != 0)) continue;
-      const float t0 = ref_term_nz(R, static_cast<long long>(di) * dr_out);
-      const float t1 = ref_term_nz(S, static_cast<long long>(di) * ds_out);
-      const float t2 = ref_term_nz(Rc, static_cast<long long>(dn) * dr_in);
-      const float t3 = ref_term_nz(Sc, static_cast<long long>(dn) * ds_in);
-      dS = ref32_accumulate<G>(g, dS, t0, t1, t2, t3, false, buf);
+      if (!__any_sync(0xffffffffu, (R | S | Rc | Sc) != 0)) continue;
+      const float t0 = ref_term_nz(R, di, dor);
+      const float t1 = ref_term_nz(S, di, dos);
+      const float t2 = ref_term_nz(Rc, dn, dir);
+      const float t3 = ref_term_nz(Sc, dn, dis);
+      dS = ref32_accumulate<G>(dS, g.gl, t0, t1, t2, t3, false, buf);
     }
   }
-  const int dor_n = dr_out - kout, dos_n = ds_out + kout;
-  const int dir_n = dr_in - kin, dis_n = ds_in + kin;
-  const int rr_r = Rr - wor, rr_s = Rs - wos, sr_r = Sr + wor, sr_s = Ss + wos;
-  if (rr_r) dS = __fsub_rn(dS, ref_term(rr_r, static_cast<long long>(dir_n) * dor_n));
-  if (rr_s) dS = __fsub_rn(dS, ref_term(rr_s, static_cast<long long>(dis_n) * dor_n));
-  if (sr_r) dS = __fsub_rn(dS, ref_term(sr_r, static_cast<long long>(dir_n) * dos_n));
-  if (sr_s) dS = __fsub_rn(dS, ref_term(sr_s, static_cast<long long>(dis_n) * dos_n));
+  dS = ref32_corner(dS, q);
+  const float dor_n = q.fn.x, dos_n = q.fn.y, dir_n = q.fn.z, dis_n = q.fn.w;
   auto nload = [&](int i) {
     nR = nS = nRc = nSc = ndi = ndn = 0;
     if (i < B && i != r && i != s) {
@@ -598,7 +664,7 @@ __device__ __noinline__ float ref32_nodal(const Ops ops, const int32_t* __restri
   nload(g.gl);
   for (int base = 0; base < B; base += G) {
     int R = nR, S = nS, Rc = nRc, Sc = nSc;
-    const int di = ndi, dn = ndn;
+    const float di = __int2float_rn(ndi), dn = __int2float_rn(ndn);
     nload(base + G + g.gl);
     const int i = base + g.gl;
     // v's edges towards block i are part of M[r,i] (out) and M[i,r] (in)
@@ -612,16 +678,160 @@ __device__ __noinline__ float ref32_nodal(const Ops ops, const int32_t* __restri
       Rc -= w;
       Sc += w;
     }
-    if (!g.any((R | S | Rc | Sc) != 0)) continue;
+    if (!__any_sync(0xffffffffu, (R | S | Rc | Sc) != 0)) continue;
     // (all four evaluated, the empty ones discarded: no branches, so the
     // four evaluations overlap)
-    const float u0 = ref_term_nz(R, static_cast<long long>(di) * dor_n);
-    const float u1 = ref_term_nz(S, static_cast<long long>(di) * dos_n);
-    const float u2 = ref_term_nz(Rc, static_cast<long long>(dn) * dir_n);
-    const float u3 = ref_term_nz(Sc, static_cast<long long>(dn) * dis_n);
-    dS = ref32_accumulate<G>(g, dS, u0, u1, u2, u3, true, buf);
+    const float u0 = ref_term_nz(R, di, dor_n);
+    const float u1 = ref_term_nz(S, di, dos_n);
+    const float u2 = ref_term_nz(Rc, dn, dir_n);
+    const float u3 = ref_term_nz(Sc, dn, dis_n);
+    dS = ref32_accumulate<G>(dS, g.gl, u0, u1, u2, u3, true, buf);
   }
   return dS;
+}
+
+// --- the same float dS on a sparse tile -----------------------------------------
+// One proposal by a whole warp.  The rows are read 64 blocks at a time (two
+// per lane), the non-zero entries of the four rows are packed into the
+// warp's queue in the chain's order, and whenever 32 are queued each lane
+// evaluates one term: empty cells cost a compare instead of a term and four
+// additions.
+constexpr int kQueueInts = 2 * (32 + 256) + 32;   // the queue, then a run's terms
+constexpr int kQueue = 32 + 256;   // entries: fewer than 32 left over, and up to 256 of 64 blocks
+
+// a run of 32 (or, at the end, n < 32) terms added to or subtracted from the chain
+__device__ __forceinline__ float ref32_run(float dS, float t, bool sub, float* buf, int lane) {
+  buf[lane] = t;
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const float4 x = reinterpret_cast<const float4*>(buf)[j];
+    if (sub) dS = __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(dS, x.x), x.y), x.z), x.w);
+    else dS = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(dS, x.x), x.y), x.z), x.w);
+  }
+  __syncwarp();
+  return dS;
+}
+
+// One pass (old-state terms added, or new-state terms subtracted) over the
+// rows.  An entry
+// holds the count and, for its row's factor, the block's degree (below
+// 2^24) with the row's number above it.
+template <class Ops, bool kNew>
+__device__ __forceinline__ float ref32_sparse_pass(float dS, const Ops& ops, const int32_t* __restrict__ din_p,
+                                                   const int32_t* __restrict__ dout_p, const Pend& q,
+                                                   const int* key, const int* two, const int* twi, int2* queue,
+                                                   float* buf, int lane) {
+  using LDT = typename Ops::LdT;
+  const int B = ops.B, r = q.r, s = q.s;
+  const int cap = q.cap, lg = q.lg;
+  const float4 ff = kNew ? q.fn : q.fo;
+  const int* mr = ops.v.M + static_cast<long long>(r) * ops.v.ld;
+  const int* ms = ops.v.M + static_cast<long long>(s) * ops.v.ld;
+  const int* tr = ops.v.Mt + static_cast<long long>(r) * ops.v.ld;
+  const int* ts = ops.v.Mt + static_cast<long long>(s) * ops.v.ld;
+  int2 nx[6];
+  auto load = [&](int i) {
+    const int2 z = make_int2(0, 0);
+    const bool in = i < B;   // rows are padded to an even number of columns with zeros
+    nx[0] = in ? LDT::ld(reinterpret_cast<const int2*>(mr + i)) : z;
+    nx[1] = in ? LDT::ld(reinterpret_cast<const int2*>(ms + i)) : z;
+    nx[2] = in ? LDT::ld(reinterpret_cast<const int2*>(tr + i)) : z;
+    nx[3] = in ? LDT::ld(reinterpret_cast<const int2*>(ts + i)) : z;
+    // (the degree arrays are only as long as there are blocks)
+    nx[4] = in ? make_int2(LDT::ld(din_p + i), i + 1 < B ? LDT::ld(din_p + i + 1) : 0) : z;
+    nx[5] = in ? make_int2(LDT::ld(dout_p + i), i + 1 < B ? LDT::ld(dout_p + i + 1) : 0) : z;
+  };
+  int queued = 0;
+  auto run = [&](int head, int n) {   // the n <= 32 entries at `head`
+    int2 e = make_int2(0, 0);
+    if (lane < n) e = queue[head + lane];
+    const int j = e.y >> 24;
+    const float fa = (j & 1) ? ff.y : ff.x, fb = (j & 1) ? ff.w : ff.z;
+    dS = ref32_run(dS, ref_term_nz(e.x, __int2float_rn(e.y & 0xffffff), (j & 2) ? fb : fa), kNew, buf, lane);
+  };
+  load(2 * lane);
+  for (int base = 0; base < B; base += 64) {
+    const int i = base + 2 * lane;
+    int x[8] = {nx[0].x, nx[1].x, nx[2].x, nx[3].x, nx[0].y, nx[1].y, nx[2].y, nx[3].y};
+    const int di[2] = {nx[4].x, nx[4].y}, dn[2] = {nx[5].x, nx[5].y};
+    load(i + 64);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      const bool rs = i + k == r || i + k == s;   // columns (new: rows too) skip blocks r and s
+      if (rs) x[4 * k + 2] = x[4 * k + 3] = 0;
+      if (kNew) {
+        if (rs) x[4 * k] = x[4 * k + 1] = 0;
+        // v's edges towards block i are part of M[r,i] (out) and M[i,r] (in)
+        if (x[4 * k] > 0) {
+          const int w = table_lookup_wo(key, two, cap, lg, i + k);
+          x[4 * k] -= w;
+          x[4 * k + 1] += w;
+        }
+        if (x[4 * k + 2] > 0) {
+          const int w = table_lookup_wo(key, twi, cap, lg, i + k);
+          x[4 * k + 2] -= w;
+          x[4 * k + 3] += w;
+        }
+      }
+    }
+    int cnt = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) cnt += x[k] != 0;
+    if (!__any_sync(0xffffffffu, cnt != 0)) continue;
+    const int incl = warp_incl_scan(cnt, lane);
+    int at = queued + incl - cnt;
+    if (cnt) {
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        if (x[4 * k]) queue[at++] = make_int2(x[4 * k], di[k]);
+        if (x[4 * k + 1]) queue[at++] = make_int2(x[4 * k + 1], di[k] | 1 << 24);
+        if (x[4 * k + 2]) queue[at++] = make_int2(x[4 * k + 2], dn[k] | 2 << 24);
+        if (x[4 * k + 3]) queue[at++] = make_int2(x[4 * k + 3], dn[k] | 3 << 24);
+      }
+    }
+    queued += __shfl_sync(0xffffffffu, incl, 31);
+    __syncwarp();
+    int head = 0;
+    for (; queued - head >= 32; head += 32) run(head, 32);
+    if (head) {   // the rest to the front
+      queued -= head;
+      int2 e = make_int2(0, 0);
+      if (lane < queued) e = queue[head + lane];
+      __syncwarp();
+      if (lane < queued) queue[lane] = e;
+      __syncwarp();
+    }
+  }
+  if (queued) run(0, queued);
+  return dS;
+}
+
+template <class Ops>
+__device__ __noinline__ float ref32_sparse(const Ops ops, const int32_t* __restrict__ din_p,
+                                           const int32_t* __restrict__ dout_p, const Pend& q, const int* key,
+                                           const int* two, const int* twi, int2* queue, float* buf) {
+  const int lane = threadIdx.x & 31;
+  float dS = ref32_sparse_pass<Ops, false>(0.0f, ops, din_p, dout_p, q, key, two, twi, queue, buf, lane);
+  dS = ref32_corner(dS, q);
+  return ref32_sparse_pass<Ops, true>(dS, ops, din_p, dout_p, q, key, two, twi, queue, buf, lane);
+}
+
+template <class Ops>
+constexpr bool kHasTile = false;
+template <class L, int P, class T>
+constexpr bool kHasTile<DenseOpsT<L, P, T>> = true;
+
+// The float dS of a proposal by a whole warp, hashed neighbour blocks.  buf:
+// 128 floats (a dense tile); queue: kQueueInts ints (a sparse one).
+template <class Ops>
+__device__ __forceinline__ float ref32_eval(const NodalArgs& a, const Ops& ops, const Pend& q, const int* key,
+                                            const int* two, const int* twi, int2* queue, float* buf) {
+  if constexpr (kHasTile<Ops>) {
+    if (a.sparse)
+      return ref32_sparse<Ops>(ops, a.din, a.dout, q, key, two, twi, queue, reinterpret_cast<float*>(queue + kQueue));
+  }
+  return ref32_nodal<Ops, 32>(ops, a.din, a.dout, a.Trow, a.Tcol, a.tld, q, key, two, twi, buf);
 }
 
 // per-vertex outputs of a decided proposal; returns whether it is accepted
@@ -722,60 +932,117 @@ __device__ __forceinline__ void tally_flush(const CtaTally* t, NodalCtl* ctl) {
   f32_tally_flush(&t->f32, &ctl->f32);
 }
 
-// Proposal for one vertex of degree <= 4 * G by a group of G lanes (a
-// warp, G = 32, or a half-warp, G = 16).  Each lane loads up to four
-// neighbours at once (ids, then their blocks) and keeps them in registers:
-// the hash of neighbour blocks and the target draw (whose chosen neighbour
-// is among them) come from the same loads.  key/two/twi: the group's table
-// of 8 * G slots; list: 4 * G ints.
-template <class Ops, int G>
-__device__ __forceinline__ void group_vertex(const NodalArgs& a, const Ops& ops, int v, uint32_t itr, int* key,
-                                             int* two, int* twi, int* list, CtaTally* tl, const Grp<G>& g,
+// The outcome of a decided proposal (one lane of its group): written out,
+// tallied, and its edge chunks listed for the CTA's apply pass.
+template <class Ops>
+__device__ __forceinline__ void close_vertex(const NodalArgs& a, const Pend& q, double f, CtaTally* tl,
                                              unsigned long long* my_bytes) {
+  const bool shadow = Ops::kP != 3 || a.shadow;
+  // without the shadow the -inf of a new-state term x log(x / 0) comes
+  // from the float sum itself (the term is +inf there, and every new-state
+  // term is subtracted)
+  const int ninf = shadow ? q.ninf : (isinf(f) && f < 0.0 ? 1 : 0);
+  const bool moved = emit<Ops::kP>(a, q.v, q.r, q.s, q.acc, f, ninf);
+  tally<Ops::kP>(tl, moved, q.acc, f, ninf, shadow);
+  if (moved && tl->own && !q.hub) {
+    const int nch = q.deg > 32 ? (q.deg + 31) >> 5 : 1;   // the vertex's chunks (one even without edges)
+    const int i0 = atomicAdd(tl->nown, nch);
+    for (int c = 0; c < nch; c++)
+      if (i0 + c < tl->own_cap) tl->own[i0 + c] = make_int2(q.v, tl->own_tag | c);
+  }
+  // precision 3 also reads, for the old-state and again for the new-state
+  // terms, rows r and s and columns r and s of M and both degree arrays:
+  // 2 x 24 bytes per block, as the reference's O(B) loops do
+  if (a.stats)
+    *my_bytes += 8 + 8ull * q.deg + 48ull * q.noccupied + 48 + 8ull * q.scanned + (Ops::kP == 3 ? 48ull * a.B : 0ull);
+}
+
+// Proposal for one vertex of degree <= KN * G by a group of G lanes (a
+// warp, G = 32, or a half-warp, G = 16).  Each lane loads up to KN
+// neighbours at once (ids, then their blocks) and keeps them in registers:
+// the weights by neighbour block and the target draw (whose chosen neighbour
+// is among them) come from the same loads.  tab: the group's 24 * G ints
+// (hashed: 8 * G slots of key, out- and in-weight); list: KN * G ints.  With
+// a.hub_units a warp also takes larger degrees, in steps of KN * G
+// neighbours.  Closes the proposal, or in precision 3 leaves it in shared
+// memory (the next entry of *pl, or *slot without a list; job: its job) for
+// its float dS to be evaluated; returns whether it did.
+template <int G>
+constexpr int kGroupNbrs = G == 32 ? kHubDegree / 32 : kPairDegree / 16;
+
+template <class Ops, int G>
+__device__ __forceinline__ bool group_vertex(const NodalArgs& a, const Ops& ops, int v, uint32_t itr, int* tab,
+                                             int* list, CtaTally* tl, const Grp<G>& g, unsigned long long* my_bytes,
+                                             Pend* slot, PendList* pl, int job) {
   using LD = typename Ops::Ld;
   using LDT = typename Ops::LdT;
-  constexpr int KN = 4;   // neighbours per lane
+  constexpr int KN = kGroupNbrs<G>;
+  int *key = tab, *two = tab + 8 * G, *twi = tab + 16 * G;
   const unsigned lanes_below = (1u << g.gl) - 1u;
   const VertexInfo vi = vertex_info<Ops>(a, v);
   const int deg = vi.dego + vi.degi;
-  if (deg > KN * G) return;   // proposed by a larger group or a whole CTA
+  const bool big = deg > KN * G;
+  if (big && !(Ops::kP == 3 && G == 32 && a.hub_units)) return false;   // proposed by a larger group or a whole CTA
   const int r = vi.r;
   const Draws x = philox(static_cast<uint32_t>(v), itr, a.stage, kTagNodal, a.seed);
   const long long dr_out = LDT::ld(a.dout + r), dr_in = LDT::ld(a.din + r);
+  int mode = kNbrHash;
+  if (Ops::kP == 3 && a.coop && !a.shadow) {
+    if (a.unit && deg <= 255 && a.B <= 48 * G) mode = kNbr8;
+    else if (a.B <= 24 * G && vi.kout < 65536 && vi.kin < 65536) mode = kNbr16;
+  }
+  // at most 8 * G slots, of which a quarter stays free (deg <= 6 * G)
   int lg = 5;
-  while ((1 << lg) < 2 * deg) lg++;
-  const int cap = 1 << lg;   // <= 8 * G
-  for (int i = g.gl; i < cap; i += G) {
-    key[i] = -1;
-    two[i] = 0;
-    twi[i] = 0;
+  while ((1 << lg) < 2 * deg && (1 << lg) < 8 * G) lg++;
+  const int cap = 1 << lg;
+  if (mode == kNbrHash) {
+    for (int i = g.gl; i < cap; i += G) {
+      key[i] = -1;
+      two[i] = 0;
+      twi[i] = 0;
+    }
+  } else {
+    const int words = mode == kNbr8 ? (a.B + 1) >> 1 : a.B;
+    for (int i = g.gl; i < words; i += G) tab[i] = 0;
   }
   g.sync();
+  auto insert = [&](int b, int w, bool is_out) {
+    if (mode == kNbrHash) table_insert(key, two, twi, cap, lg, b, w, is_out);
+    else if (mode == kNbr8) atomicAdd(reinterpret_cast<unsigned*>(tab) + (b >> 1), 1u << (((b & 1) << 4) | (is_out ? 0 : 8)));
+    else atomicAdd(reinterpret_cast<unsigned*>(tab) + b, static_cast<unsigned>(w) << (is_out ? 0 : 16));
+  };
   int nb[KN], wv[KN], pb[KN];
+  // neighbours j0 + gl + G k of the out-list followed by the in-list
+  auto load_nbrs = [&](int j0) {
 #pragma unroll
-  for (int k = 0; k < KN; k++) {
-    const int j = g.gl + G * k;
-    nb[k] = 0;
-    wv[k] = 0;
-    if (j < deg) {
-      const bool is_out = j < vi.dego;
-      nb[k] = is_out ? __ldg(a.out_idx + vi.o0 + j) : __ldg(a.in_idx + vi.i0 + j - vi.dego);
-      wv[k] = a.unit ? 1 : (is_out ? __ldg(a.out_w + vi.o0 + j) : __ldg(a.in_w + vi.i0 + j - vi.dego));
+    for (int k = 0; k < KN; k++) {
+      const int j = j0 + g.gl + G * k;
+      nb[k] = 0;
+      wv[k] = 0;
+      if (j < deg) {
+        const bool is_out = j < vi.dego;
+        nb[k] = is_out ? __ldg(a.out_idx + vi.o0 + j) : __ldg(a.in_idx + vi.i0 + j - vi.dego);
+        wv[k] = a.unit ? 1 : (is_out ? __ldg(a.out_w + vi.o0 + j) : __ldg(a.in_w + vi.i0 + j - vi.dego));
+      }
     }
-  }
 #pragma unroll
-  for (int k = 0; k < KN; k++) pb[k] = g.gl + G * k < deg ? LD::ld(a.part + nb[k]) : 0;
+    for (int k = 0; k < KN; k++) pb[k] = j0 + g.gl + G * k < deg ? LD::ld(a.part + nb[k]) : 0;
 #pragma unroll
-  for (int k = 0; k < KN; k++) {
-    const int j = g.gl + G * k;
-    if (j < deg) table_insert(key, two, twi, cap, lg, pb[k], wv[k], j < vi.dego);
-  }
+    for (int k = 0; k < KN; k++) {
+      const int j = j0 + g.gl + G * k;
+      if (j < deg) insert(pb[k], wv[k], j < vi.dego);
+    }
+  };
+  load_nbrs(0);
   // the target: neighbour position j by weight, its block from registers
   int scanned = 0;
   int s;
   const long long ktot = vi.kout + vi.kin;
   if (ktot == 0) {
     s = static_cast<int>(draw_below(x.x2, a.B));
+  } else if (Ops::kP == 3 && G == 32 && big) {
+    for (int j0 = KN * G; j0 < deg; j0 += KN * G) load_nbrs(j0);
+    s = propose_target(a, ops, x, vi, g.gl, &scanned);
   } else {
     const long long t = draw_below(x.x0, ktot);
     int j;
@@ -799,7 +1066,9 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, const Ops& ops,
       }
     }
     const int kq = j / G;
-    const int pj = kq == 0 ? pb[0] : kq == 1 ? pb[1] : kq == 2 ? pb[2] : pb[3];
+    int pj = pb[0];
+#pragma unroll
+    for (int k = 1; k < KN; k++) pj = kq == k ? pb[k] : pj;
     s = target_from(a, ops, x, g.shfl(pj, j & (G - 1)), g, &scanned);
   }
   g.sync();
@@ -809,7 +1078,7 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, const Ops& ops,
       if (a.stats) *my_bytes += 8 + 8ull * deg + 8ull * scanned;
     }
     g.sync();
-    return;
+    return false;
   }
   const long long ds_out = LDT::ld(a.dout + s), ds_in = LDT::ld(a.din + s);
   int e4 = 0;
@@ -836,11 +1105,11 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, const Ops& ops,
       noccupied += __popc(occ);
     }
     g.sync();
-    // each lane has at most four slots (nlist <= 4 * G): their M entries
-    // and degrees are loaded in two rounds of two, then the log terms
+    // each lane has at most KN slots (nlist <= KN * G): their M entries
+    // and degrees are loaded in rounds of two, then the log terms
     TermSums ts{0, 0, 0, 0, 0};
 #pragma unroll
-    for (int k0 = 0; k0 < 4; k0 += 2) {
+    for (int k0 = 0; k0 < KN; k0 += 2) {
       int R[2], S[2], Rc[2], Sc[2], Di[2], Do[2], wo[2], wi[2];
 #pragma unroll
       for (int k = 0; k < 2; k++) {
@@ -880,58 +1149,88 @@ __device__ __forceinline__ void group_vertex(const NodalArgs& a, const Ops& ops,
                                    vi.kin, &ninf, ts.f, &f);
   }
   if constexpr (Ops::kP == 3) {
-    const int Rr = g.shfl(e4, 0), Rs = g.shfl(e4, 1);
-    const int Sr = g.shfl(e4, 2), Ss = g.shfl(e4, 3);
-    const int wor = table_lookup_wo(key, two, cap, lg, r);
-    const int wos = table_lookup_wo(key, two, cap, lg, s);
-    f = ref32_nodal<Ops, G>(ops, a.din, a.dout, a.Trow, a.Tcol, a.tld, r, s, static_cast<int>(dr_out),
-                            static_cast<int>(dr_in),
-                            static_cast<int>(ds_out), static_cast<int>(ds_in), static_cast<int>(vi.kout),
-                            static_cast<int>(vi.kin), static_cast<int>(Rr), static_cast<int>(Rs),
-                            static_cast<int>(Sr), static_cast<int>(Ss), static_cast<int>(wor),
-                            static_cast<int>(wos), key, two, twi, cap, lg, reinterpret_cast<float*>(list));
-    // without the shadow the -inf of a new-state term x log(x / 0) comes
-    // from the float sum itself (the term is +inf there, and every new-state
-    // term is subtracted)
-    if (!shadow) ninf = isinf(f) && f < 0.0 ? 1 : 0;
-  }
-  if (g.gl == 0) {
-    const bool moved = emit<Ops::kP>(a, v, r, s, acc, f, ninf);
-    tally<Ops::kP>(tl, moved, acc, f, ninf, shadow);
-    if (moved && tl->own) {
-      const int nch = deg > 32 ? (deg + 31) >> 5 : 1;   // the vertex's chunks (one even without edges)
-      const int i0 = atomicAdd(tl->nown, nch);
-      for (int c = 0; c < nch; c++)
-        if (i0 + c < tl->own_cap) tl->own[i0 + c] = make_int2(v, tl->own_tag | c);
+    const int e0 = g.shfl(e4, 0), e1 = g.shfl(e4, 1), e2 = g.shfl(e4, 2), e3 = g.shfl(e4, 3);
+    if (g.gl == 0) {
+      Pend& q = pl ? pl->p[atomicAdd(&pl->n, 1)] : *slot;
+      q.mode = mode;
+      q.hub = false;
+      q.job = job;
+      q.tab = key;
+      q.two = two;
+      q.twi = twi;
+      q.v = v;
+      q.r = r;
+      q.s = s;
+      q.deg = deg;
+      q.scanned = scanned;
+      q.noccupied = noccupied;
+      q.acc = acc;
+      q.ninf = ninf;
+      q.cap = cap;
+      q.lg = lg;
+      q.dr_out = static_cast<int>(dr_out);
+      q.dr_in = static_cast<int>(dr_in);
+      q.ds_out = static_cast<int>(ds_out);
+      q.ds_in = static_cast<int>(ds_in);
+      q.kout = static_cast<int>(vi.kout);
+      q.kin = static_cast<int>(vi.kin);
+      q.Rr = e0;
+      q.Rs = e1;
+      q.Sr = e2;
+      q.Ss = e3;
+      int unused;
+      nbr_weights(q, r, &q.wor, &unused);
+      nbr_weights(q, s, &q.wos, &unused);
+      set_factors(q);
     }
-    // precision 3 also reads, for the old-state and again for the new-state
-    // terms, rows r and s and columns r and s of M and both degree arrays:
-    // 2 x 24 bytes per block, as the reference's O(B) loops do
-    if (a.stats)
-      *my_bytes += 8 + 8ull * deg + 48ull * noccupied + 48 + 8ull * scanned + (Ops::kP == 3 ? 48ull * a.B : 0ull);
+    g.sync();
+    return true;
+  } else {
+    Pend q{};
+    q.v = v;
+    q.r = r;
+    q.s = s;
+    q.deg = deg;
+    q.scanned = scanned;
+    q.noccupied = noccupied;
+    q.acc = acc;
+    q.ninf = ninf;
+    if (g.gl == 0) close_vertex<Ops>(a, q, f, tl, my_bytes);
+    g.sync();
+    return false;
   }
-  g.sync();
 }
 
 // One warp per vertex of degree <= kHubDegree; 5 CTAs per SM so that a
 // batch of the bench workload (N/10 = 5000 vertices) runs in one wave.
 template <class Ops>
 __global__ void __launch_bounds__(kThreads, 5) k_nodal_propose(NodalArgs a, Ops ops) {
-  __shared__ int s_key[kWarps][kHCap];
-  __shared__ int s_wo[kWarps][kHCap];
-  __shared__ int s_wi[kWarps][kHCap];
-  __shared__ __align__(16) int s_list[kWarps][kHubDegree];   // occupied slots other than r, s; then the float dS's terms
+  __shared__ int s_tab[kWarps][3 * kHCap];
+  // occupied slots other than r, s; then the float dS's terms, or its queue
+  __shared__ __align__(16) int s_list[kWarps][kQueueInts];
+  __shared__ Pend s_pend[Ops::kP == 3 ? kWarps : 1];
   __shared__ CtaTally s_tally;
   if (a.ctl->done) return;   // written by earlier launches only
   const uint32_t itr = static_cast<uint32_t>(a.ctl->itr);
   if (threadIdx.x == 0) s_tally = CtaTally{0, 0, 0, 0};
+  if constexpr (Ops::kP == 3) ref_tab_fill();
   __syncthreads();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int nwarps = gridDim.x * kWarps;
   unsigned long long my_bytes = 0;
-  for (int v = a.beg + blockIdx.x * kWarps + wib; v < a.end; v += nwarps)
-    group_vertex(a, ops, v, itr, s_key[wib], s_wo[wib], s_wi[wib], s_list[wib], &s_tally, Grp<32>(lane),
-                 &my_bytes);
+  for (int v = a.beg + blockIdx.x * kWarps + wib; v < a.end; v += nwarps) {
+    int* const tab = s_tab[wib];
+    const bool live = group_vertex(a, ops, v, itr, tab, s_list[wib], &s_tally, Grp<32>(lane), &my_bytes,
+                                   Ops::kP == 3 ? s_pend + wib : nullptr, nullptr, 0);
+    if constexpr (Ops::kP == 3) {
+      if (live) {   // warp-uniform
+        const float f = ref32_eval(a, ops, s_pend[wib], tab, tab + kHCap, tab + 2 * kHCap,
+                                   reinterpret_cast<int2*>(s_list[wib]), reinterpret_cast<float*>(s_list[wib]));
+        if (lane == 0) close_vertex<Ops>(a, s_pend[wib], f, &s_tally, &my_bytes);
+        __syncwarp();
+      }
+    }
+  }
   __syncthreads();
   if (threadIdx.x == 0) tally_flush(&s_tally, a.ctl);
   if (a.stats && lane == 0 && my_bytes) atomicAdd(&a.ctl->bytes, my_bytes);
@@ -943,18 +1242,22 @@ struct HubShared {
   int sum[5][NW];
   float fhi[NW], flo[NW];   // FP32 partial sums (precision modes 1, 2)
   int target, scanned;
-  __align__(16) float chain[128];   // precision 3: the float dS's staged terms (warp 0)
+  Pend pend;   // precision 3, without a list
 };
 
 // Proposal for one vertex of degree > kHubDegree by a whole CTA of NT
 // threads.  The last warp draws the target while the others fill the hash
 // of neighbour blocks (at most min(deg, B) entries: in `stab`, a shared
 // region of `scap` slots per array, or beyond that in the vertex's global
-// region); each thread loads four neighbours at once, and up to four
-// occupied slots at once for the terms.
+// region; with a list, precision 3, the arrays follow one another from the
+// region's end); each thread loads four neighbours at once, and up to four
+// occupied slots at once for the terms.  In precision 3 the proposal is left
+// in pl's first entry (as job `job`), or, without a list, warp 0 evaluates
+// its float dS (chain: kQueueInts ints).
 template <class Ops, int NT>
 __device__ __forceinline__ void hub_vertex(const NodalArgs& a, const Ops& ops, int v, uint32_t itr, int* stab,
-                                           int scap, HubShared<NT / 32>* sh, unsigned long long* my_bytes) {
+                                           int scap, HubShared<NT / 32>* sh, unsigned long long* my_bytes,
+                                           int* chain, PendList* pl, int job) {
   using LD = typename Ops::Ld;
   using LDT = typename Ops::LdT;
   constexpr int NW = NT / 32;
@@ -972,6 +1275,11 @@ __device__ __forceinline__ void hub_vertex(const NodalArgs& a, const Ops& ops, i
     key = stab;
     two = stab + scap;
     twi = stab + 2 * scap;
+    if (Ops::kP == 3 && pl) {   // what precedes them is free for the float dS
+      key = stab + 3 * (scap - cap);
+      two = key + cap;
+      twi = two + cap;
+    }
   } else {
     const long long off = __ldg(a.hi_off + v);
     key = a.hkey + off;
@@ -1097,19 +1405,50 @@ __device__ __forceinline__ void hub_vertex(const NodalArgs& a, const Ops& ops, i
     double f = 0.0;
     const long long acc = finalize_grp<32, Ops::kP>(a, Grp<32>(lane), tot, Rr, Rs, Sr, Ss, wor, wos, dr_out,
                                                     dr_in, ds_out, ds_in, vi.kout, vi.kin, &ninf, fpart, &f);
-    if constexpr (Ops::kP == 3)
-      f = ref32_nodal<Ops, 32>(ops, a.din, a.dout, a.Trow, a.Tcol, a.tld, r, s, static_cast<int>(dr_out),
-                               static_cast<int>(dr_in),
-                               static_cast<int>(ds_out), static_cast<int>(ds_in), static_cast<int>(vi.kout),
-                               static_cast<int>(vi.kin), static_cast<int>(Rr), static_cast<int>(Rs),
-                               static_cast<int>(Sr), static_cast<int>(Ss), static_cast<int>(wor),
-                               static_cast<int>(wos), key, two, twi, cap, lg, sh->chain);
+    if constexpr (Ops::kP == 3) {
+      Pend& q = pl ? pl->p[0] : sh->pend;
+      if (lane == 0) {
+        q.mode = kNbrHash;
+        q.hub = true;
+        q.job = job;
+        q.tab = key;
+        q.two = two;
+        q.twi = twi;
+        q.v = v;
+        q.deg = deg;
+        q.scanned = sh->scanned;
+        q.noccupied = occ;
+        q.acc = acc;
+        q.ninf = ninf;
+        q.r = r;
+        q.s = s;
+        q.dr_out = static_cast<int>(dr_out);
+        q.dr_in = static_cast<int>(dr_in);
+        q.ds_out = static_cast<int>(ds_out);
+        q.ds_in = static_cast<int>(ds_in);
+        q.kout = static_cast<int>(vi.kout);
+        q.kin = static_cast<int>(vi.kin);
+        q.Rr = static_cast<int>(Rr);
+        q.Rs = static_cast<int>(Rs);
+        q.Sr = static_cast<int>(Sr);
+        q.Ss = static_cast<int>(Ss);
+        q.wor = static_cast<int>(wor);
+        q.wos = static_cast<int>(wos);
+        q.cap = cap;
+        q.lg = lg;
+        set_factors(q);
+        if (pl) pl->n = 1;
+      }
+      __syncwarp();
+      if (!pl)
+        f = ref32_eval(a, ops, q, key, two, twi, reinterpret_cast<int2*>(chain), reinterpret_cast<float*>(chain));
+    }
     // (a hub's exact value is a CTA-parallel sum over its slots and is
     // always evaluated; without the shadow it is not reported, as for the
     // other vertices)
     const bool shadow = Ops::kP != 3 || a.shadow;
     if (!shadow) ninf = isinf(f) && f < 0.0 ? 1 : 0;
-    if (lane == 0) {
+    if (lane == 0 && !(Ops::kP == 3 && pl)) {
       tally_ctl<Ops::kP>(a.ctl, emit<Ops::kP>(a, v, r, s, acc, f, ninf), acc, f, ninf, shadow);
       if (a.stats)
         *my_bytes += 8 + 8ull * deg + 48ull * occ + 48 + 8ull * sh->scanned + (Ops::kP == 3 ? 48ull * a.B : 0ull);
@@ -1125,11 +1464,16 @@ __global__ void __launch_bounds__(kHubThreads) k_nodal_propose_hub(NodalArgs a, 
                                                                   int hub_lo, int hub_hi, int smem_cap) {
   extern __shared__ __align__(16) int dyn[];
   __shared__ HubShared<kHubWarps> sh;
+  __shared__ __align__(16) int s_chain[Ops::kP == 3 ? kQueueInts : 1];
   if (a.ctl->done) return;
   const uint32_t itr = static_cast<uint32_t>(a.ctl->itr);
   unsigned long long my_bytes = 0;
+  if constexpr (Ops::kP == 3) {
+    ref_tab_fill();
+    __syncthreads();
+  }
   for (int h = hub_lo + blockIdx.x; h < hub_hi; h += gridDim.x)
-    hub_vertex<Ops, kHubThreads>(a, ops, __ldg(hubs + h), itr, dyn, smem_cap, &sh, &my_bytes);
+    hub_vertex<Ops, kHubThreads>(a, ops, __ldg(hubs + h), itr, dyn, smem_cap, &sh, &my_bytes, s_chain, nullptr, 0);
   if (a.stats && threadIdx.x == 0 && my_bytes) atomicAdd(&a.ctl->bytes, my_bytes);
 }
 
@@ -1625,23 +1969,26 @@ __global__ void k_ctl_sweep_start(NodalCtl* ctl, int W, const long long* ide_q,
 // --- persistent nodal phase ----------------------------------------------------
 constexpr int kPThreads = 768;    // one CTA per SM (80 registers a thread)
 constexpr int kPWarps = kPThreads / 32;
-constexpr int kUnitWarp = -2;     // work unit of one vertex with 64 < degree <= 128
+constexpr int kUnitWarp = -2;     // work unit of one vertex of degree <= kHubDegree
 constexpr int kPHubLg = 13;
 constexpr int kPHubSlots = 1 << kPHubLg;  // hub table slots in shared memory; larger hub tables are global
 constexpr int kDeltaGlobalMinB = 256;     // from this B the phase kernel's apply writes straight to global memory
-// the proposals of the phase kernel read the tile from shared memory up to
-// this B: M and Mt (B x ld each, ld = B rounded up to 4) after the first
-// kSnapOff slots of the hub table's first and second arrays, chunk sums and
-// degrees after those of its third
+// The proposals of the phase kernel read the tile from shared memory up to
+// this B: after a hub table of kSnapSlots slots per array come M and Mt (B x
+// ld each, ld = B rounded up to 4), chunk sums and degrees; the rest of the
+// hub region stages the cooperative float dS
 constexpr int kSnapMaxB = 88;
-constexpr int kSnapOff = 256;   // >= a hub table's capacity for B <= kSnapMaxB (2 * B rounded up to a power of 2)
-static_assert(kSnapOff + kSnapMaxB * ((kSnapMaxB + 3) & ~3) <= kPHubSlots, "tile copy overruns its region");
-static_assert(kSnapOff + 3 * kSnapMaxB <= kPHubSlots, "degree copy overruns its region");
-static_assert(2 * kSnapMaxB <= kSnapOff && kSnapMaxB <= kChunk, "hub tables or chunk sums outgrow the layout");
-static_assert(kPHubSlots == kPhaseHubSlots, "hub regions are assigned for tables beyond this size");
+constexpr int kSnapSlots = 256;   // >= a hub table's capacity for B <= kSnapMaxB (2 * B rounded up to a power of 2)
+static_assert(kMaxPend == 2 * kPWarps, "a wave's proposals outgrow the list");
+static_assert(3 * kSnapSlots + 2 * kSnapMaxB * kSnapMaxB + 3 * kSnapMaxB + 2 * kMaxPend * (4 * 16 + 4) <= 3 * kPHubSlots,
+              "chunks of 16 blocks of a full list fit beside the tile copy");
+static_assert(2 * kSnapMaxB <= kSnapSlots && kSnapMaxB <= kChunk, "hub tables or chunk sums outgrow the layout");
+static_assert(kPHubSlots == 2 * kPhaseHubSlots, "hub regions are assigned for tables beyond this size");
 constexpr unsigned long long kBarrierTimeoutNs = 200ull * 1000ull * 1000ull;
 // dynamic shared memory: per-warp tables and lists, then the hub table
 constexpr size_t kPWarpInts = 3 * kHCap + kHubDegree;
+static_assert(kMaxPend <= kMaxSlots && 2 * kMaxSlots * kSlot <= 3 * kPHubSlots,
+              "a step of a full list on a sparse tile outgrows the hub region");
 constexpr size_t kPSmemBytes = sizeof(int) * (kPWarps * kPWarpInts + 3 * kPHubSlots);
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -1742,24 +2089,351 @@ __device__ __forceinline__ unsigned long long apply_bytes(const NodalArgs& a, in
                   (__ldg(a.in_ptr + ch.x + 1) - __ldg(a.in_ptr + ch.x));
   return 24ull * static_cast<unsigned long long>(max(0, min(32, deg - 32 * ch.y)));
 }
+// --- float dS of a CTA's proposals, evaluated together ---------------------------
+// Every proposal needs up to 8 B terms added one after the other: evaluating
+// a term takes about 60 issue slots a warp, adding it 4 cycles of one thread's
+// dependent latency.  All warps but one evaluate terms, for a chunk of blocks
+// of every proposal at a time, into one of two staging areas in shared
+// memory, while the last warp, a thread per proposal, adds the chunk before.
+// So the additions of up to 32 chains issue together (a warp per chain
+// repeats its additions in every lane), the work of a wave is spread over the
+// CTA whatever its number of proposals, and a small batch has 23 warps on its
+// few.  It is bound by the issue of the evaluating warps; with few proposals
+// and a large B by the chain.  A batch of N = 50000 (34 proposals a CTA) took
+// 69 us at B = 382 against 143 us with a chain per half-warp, 27 us against
+// 35 us at B = 48; one of N = 5000 (8 a CTA) 28 us against 37 us at B = 151.
+
+// the four terms of block i of proposal q, old-state or new-state
+template <class Ops>
+__device__ __forceinline__ float4 coop_cell(const NodalArgs& a, const Ops& ops, const Pend& q, int i, bool fresh) {
+  using LDT = typename Ops::LdT;
+  const bool rs = i == q.r || i == q.s;
+  if (!fresh && a.Trow) {
+    const long long ro = static_cast<long long>(q.r) * a.tld + i, so = static_cast<long long>(q.s) * a.tld + i;
+    return make_float4(__ldcg(a.Trow + ro), __ldcg(a.Trow + so), rs ? 0.0f : __ldcg(a.Tcol + ro),
+                       rs ? 0.0f : __ldcg(a.Tcol + so));
+  }
+  if (fresh && rs) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  int R = ops.get(q.r, i), S = ops.get(q.s, i), Rc = 0, Sc = 0;
+  if (!rs) {   // columns skip i in {r, s}
+    Rc = ops.get_t(q.r, i);
+    Sc = ops.get_t(q.s, i);
+  }
+  const float di = __int2float_rn(LDT::ld(a.din + i)), dn = __int2float_rn(LDT::ld(a.dout + i));
+  const float4 f = fresh ? q.fn : q.fo;
+  if (fresh) {   // v's edges towards block i are part of M[r,i] (out) and M[i,r] (in)
+    int wo, wi;
+    nbr_weights(q, i, &wo, &wi);
+    R -= wo;
+    S += wo;
+    Rc -= wi;
+    Sc += wi;
+  }
+  return make_float4(ref_term_nz(R, di, f.x), ref_term_nz(S, di, f.y), ref_term_nz(Rc, dn, f.z),
+                     ref_term_nz(Sc, dn, f.w));
+}
+
+// The float dS of the listed proposals, handed to close(q, f) by one thread
+// each (CTA-collective).  stage: `room` floats; job: SingleJob or GangJobs.
+template <int NT, class JobFn, class CloseFn>
+__device__ __forceinline__ void coop_eval(const PendList& pl, float* stage, int room, JobFn job, CloseFn close) {
+  constexpr int NW = NT / 32;
+  const int np = pl.n;
+  if (np == 0) return;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int nc = np > 32 ? 2 : 1;        // warps that add: a proposal per lane
+  const int nprod = NT - 32 * nc;        // threads that evaluate
+  const bool adds = wib >= NW - nc;
+  const int mine = (wib - (NW - nc)) * 32 + lane;
+  int bmax = 0, bmine = 0;
+  for (int k = lane; k < np; k += 32) bmax = max(bmax, job.blocks(pl.p[k].job));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
+  // chunks of CB blocks, equal shares of the largest B: at most about four
+  // cells per evaluating thread, so that the last chunk's additions, which
+  // overlap nothing, stay short, and both buffers within the room.  (A row of
+  // the staging area is an odd number of 16-byte words: no bank conflicts
+  // among the adding lanes.)
+  const int most = max(8, min(4 * nprod / np, (room / (8 * np) - 1) & ~1));
+  const int nch = (bmax + most - 1) / most;
+  const int CB = ((bmax + nch - 1) / nch + 1) & ~1, stride = 4 * CB + 4;
+  float dS = 0.0f, c0 = 0.0f, c1 = 0.0f, c2 = 0.0f, c3 = 0.0f;
+  const bool has = adds && mine < np;
+  if (has) {
+    bmine = job.blocks(pl.p[mine].job);
+    corner_terms(pl.p[mine], &c0, &c1, &c2, &c3);   // due between the passes
+  }
+  const int dk = nprod / CB, dr = nprod - dk * CB;   // from one of a thread's cells to its next
+  for (int t = 0; t <= 2 * nch; t++) {
+    if (!adds) {
+      if (t < 2 * nch) {
+        const bool fresh = t >= nch;
+        const int b0 = (fresh ? t - nch : t) * CB;
+        float* st = stage + (t & 1) * np * stride;
+        int k = threadIdx.x / CB, o = threadIdx.x - k * CB;
+        for (; k < np;) {
+          job.cell(pl.p[k], b0 + o, fresh, reinterpret_cast<float4*>(st + k * stride + 4 * o));
+          k += dk;
+          o += dr;
+          if (o >= CB) {
+            o -= CB;
+            k++;
+          }
+        }
+      }
+    } else if (has && t > 0) {
+      const bool fresh = t > nch;
+      const int b0 = (fresh ? t - 1 - nch : t - 1) * CB;
+      const int n = min(CB, bmine - b0);
+      const float4* st = reinterpret_cast<const float4*>(stage + ((t - 1) & 1) * np * stride + mine * stride);
+      if (!fresh) {
+#pragma unroll 8
+        for (int j = 0; j < n; j++) {
+          const float4 q = st[j];
+          dS = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(dS, q.x), q.y), q.z), q.w);
+        }
+      } else {
+        if (t == nch + 1) dS = __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(dS, c0), c1), c2), c3);
+#pragma unroll 8
+        for (int j = 0; j < n; j++) {
+          const float4 q = st[j];
+          dS = __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(dS, q.x), q.y), q.z), q.w);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (has) close(pl.p[mine], dS);
+}
+
+// The same on a tile with many empty cells.  A warp takes a proposal's 64
+// blocks at a time: it packs the non-zero cells of the four rows, in the
+// chain's order, into a slot of the staging area, and its lanes then replace
+// each packed cell by its term, so an empty cell costs a compare instead of
+// a term and an addition.  A packed cell holds the count (below 2^24) under
+// its number among the 256; the block's degree comes from the lane that
+// loaded it.  The loads of a warp's next 64 blocks are issued before it works
+// on these.  Bound by the issue of the scan (about 400 slots for 64 blocks).
+// N = 4999, B = 2500 (1.3% of the cells filled): 53 us a batch against 241 us
+// with whole rows evaluated; N = 50000, B = 3052 (8%): 468 against 941 us.
+struct SlotCounts {
+  int n[2][kMaxSlots];
+};
+
+// a tile, the offsets of rows r and s in it, and the block degrees
+struct RowPtrs {
+  const int *M, *Mt, *din, *dout;
+  unsigned r, s;
+};
+
+template <int NT, class JobFn, class CloseFn>
+__device__ __forceinline__ void coop_eval_sparse(const PendList& pl, float* stage, int room, SlotCounts* sc, JobFn job,
+                                                 CloseFn close) {
+  constexpr int NW = NT / 32;
+  const int np = pl.n;
+  if (np == 0) return;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int nc = np > 32 ? 2 : 1;
+  const int pw = NW - nc;
+  const bool adds = wib >= pw;
+  const int mine = (wib - pw) * 32 + lane;
+  int bmax = 0;
+  for (int k = lane; k < np; k += 32) bmax = max(bmax, job.blocks(pl.p[k].job));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
+  const int nch = (bmax + 63) >> 6;
+  // m chunks of every proposal per step, in two sets of np * m slots
+  const int m = min(nch, max(1, min(kMaxSlots, room / (2 * kSlot)) / np));
+  const int nst = (nch + m - 1) / m, per = np * m;
+  float dS = 0.0f, c0 = 0.0f, c1 = 0.0f, c2 = 0.0f, c3 = 0.0f;
+  const bool has = adds && mine < np;
+  if (has) corner_terms(pl.p[mine], &c0, &c1, &c2, &c3);
+  // a warp's items of a step: slots wib, wib + pw, wib + 2 pw (< per); slot
+  // x is chunk x / np of the step, proposal x % np
+  int2 nx[6];
+  auto load = [&](int t, int k, int c) {
+#pragma unroll
+    for (int j = 0; j < 6; j++) nx[j] = make_int2(0, 0);
+    if (t >= 2 * nst) return;
+    const Pend& q = pl.p[k];
+    const int i = (((t >= nst ? t - nst : t) * m + c) << 6) + 2 * lane;
+    if (i >= job.blocks(q.job)) return;
+    // (rows and degree arrays are readable up to an even number of blocks)
+    const RowPtrs rp = job.rows(q);
+    nx[0] = __ldcg(reinterpret_cast<const int2*>(rp.M + (rp.r + i)));
+    nx[1] = __ldcg(reinterpret_cast<const int2*>(rp.M + (rp.s + i)));
+    nx[2] = __ldcg(reinterpret_cast<const int2*>(rp.Mt + (rp.r + i)));
+    nx[3] = __ldcg(reinterpret_cast<const int2*>(rp.Mt + (rp.s + i)));
+    nx[4] = __ldcg(reinterpret_cast<const int2*>(rp.din + i));
+    nx[5] = __ldcg(reinterpret_cast<const int2*>(rp.dout + i));
+  };
+  const unsigned lanes_below = (1u << lane) - 1u;
+  const int k0 = wib % np, step_k = pw % np, c0x = wib / np, step_c = pw / np;
+  if (!adds && wib < per) load(0, k0, c0x);
+  for (int t = 0; t <= 2 * nst; t++) {
+    if (!adds) {
+      if (t < 2 * nst) {
+        const bool fresh = t >= nst;
+        int k1 = k0, c1 = c0x;
+        for (int x = wib; x < per; x += pw) {
+          const int kx = k1, cx = c1;
+          const Pend& q = pl.p[kx];
+          const int i = (((fresh ? t - nst : t) * m + cx) << 6) + 2 * lane;
+          int c[8] = {nx[0].x, nx[1].x, nx[2].x, nx[3].x, nx[0].y, nx[1].y, nx[2].y, nx[3].y};
+          const int di0 = nx[4].x, di1 = nx[4].y, dn0 = nx[5].x, dn1 = nx[5].y;
+          k1 += step_k;
+          c1 += step_c;
+          if (k1 >= np) {
+            k1 -= np;
+            c1++;
+          }
+          if (x + pw < per) load(t, k1, c1);
+          else load(t + 1, k0, c0x);
+          if (!__any_sync(0xffffffffu, (c[0] | c[1] | c[2] | c[3] | c[4] | c[5] | c[6] | c[7]) != 0)) {
+            if (lane == 0) sc->n[t & 1][x] = 0;
+            continue;
+          }
+          const int r = q.r, s = q.s;
+#pragma unroll
+          for (int k = 0; k < 2; k++) {
+            const bool rs = i + k == r || i + k == s;   // columns (new: rows too) skip blocks r and s
+            if (rs) c[4 * k + 2] = c[4 * k + 3] = 0;
+            if (fresh) {
+              if (rs) c[4 * k] = c[4 * k + 1] = 0;
+              // v's edges towards block i are part of M[r,i] (out) and M[i,r] (in)
+              if ((c[4 * k] | c[4 * k + 2]) != 0) {
+                int wo, wi;
+                nbr_weights(q, i + k, &wo, &wi);
+                c[4 * k] -= wo;
+                c[4 * k + 1] += wo;
+                c[4 * k + 2] -= wi;
+                c[4 * k + 3] += wi;
+              }
+            }
+          }
+          int total = 0, at = 0;   // non-zero cells in all, and in the lanes below
+#pragma unroll
+          for (int k = 0; k < 8; k++) {
+            const unsigned nz = __ballot_sync(0xffffffffu, c[k] != 0);
+            total += __popc(nz);
+            at += __popc(nz & lanes_below);
+          }
+          // a slot's 16-byte words are permuted by the proposal's number, so
+          // that the adding lanes, at the same place of their slots, read
+          // different banks
+          int* slot = reinterpret_cast<int*>(stage) + ((t & 1) * per + x) * kSlot;
+          const int sw = (kx & 7) << 2;
+          {
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+              if (c[k]) slot[at++ ^ sw] = c[k] | static_cast<int>(static_cast<unsigned>(8 * lane + k) << 24);
+          }
+          __syncwarp();
+          const float4 ff = fresh ? q.fn : q.fo;
+          for (int e0 = 0; e0 < total; e0 += 32) {
+            const int e = e0 + lane;
+            const unsigned w = e < total ? slot[e ^ sw] : 0u;
+            const int from = w >> 27, k = (w >> 24) & 7, j = k & 3;   // lane, cell of the lane, row
+            const int a0 = __shfl_sync(0xffffffffu, di0, from), a1 = __shfl_sync(0xffffffffu, di1, from);
+            const int b0 = __shfl_sync(0xffffffffu, dn0, from), b1 = __shfl_sync(0xffffffffu, dn1, from);
+            const int d = (j & 2) ? ((k & 4) ? b1 : b0) : ((k & 4) ? a1 : a0);
+            const float fa = (j & 1) ? ff.y : ff.x, fb = (j & 1) ? ff.w : ff.z;
+            const float term = ref_term_nz(static_cast<int>(w & 0xffffffu), __int2float_rn(d), (j & 2) ? fb : fa);
+            if (e < ((total + 3) & ~3)) slot[e ^ sw] = __float_as_int(term);   // zeros up to a multiple of 4
+          }
+          if (lane == 0) sc->n[t & 1][x] = total;
+        }
+      }
+    } else if (has && t > 0) {
+      const bool fresh = t > nst;
+      if (t == nst + 1) dS = __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(dS, c0), c1), c2), c3);
+      const int sw = mine & 7;
+      for (int x = mine; x < per; x += np) {
+        const int n = (sc->n[(t - 1) & 1][x] + 3) >> 2;
+        const float4* st = reinterpret_cast<const float4*>(stage + (((t - 1) & 1) * per + x) * kSlot);
+        if (!fresh) {
+#pragma unroll 4
+          for (int j = 0; j < n; j++) {
+            const float4 q = st[j ^ sw];
+            dS = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(dS, q.x), q.y), q.z), q.w);
+          }
+        } else {
+#pragma unroll 4
+          for (int j = 0; j < n; j++) {
+            const float4 q = st[j ^ sw];
+            dS = __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(dS, q.x), q.y), q.z), q.w);
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (has) close(pl.p[mine], dS);
+}
+
+// what the evaluation asks of the proposals' jobs: one job, or the gang's
+template <class Ops>
+struct SingleJob {
+  const NodalArgs& a;
+  const Ops& ops;
+  __device__ __forceinline__ int blocks(int) const { return a.B; }
+  __device__ __forceinline__ RowPtrs rows(const Pend& q) const {
+    return RowPtrs{ops.v.M, ops.v.Mt, a.din, a.dout, static_cast<unsigned>(q.r) * ops.v.ld,
+                   static_cast<unsigned>(q.s) * ops.v.ld};
+  }
+  __device__ __forceinline__ void cell(const Pend& q, int i, bool fresh, float4* out) const {
+    if (i < a.B) *out = coop_cell(a, ops, q, i, fresh);
+  }
+};
+
+template <class Ops>
+struct GangJobs {
+  const PhaseArgs* jobs;
+  __device__ __forceinline__ int blocks(int j) const { return jobs[j].a.B; }
+  __device__ __forceinline__ RowPtrs rows(const Pend& q) const {
+    const PhaseArgs& p = jobs[q.job];
+    return RowPtrs{p.v.M, p.v.Mt, p.a.din, p.a.dout, static_cast<unsigned>(q.r) * p.v.ld,
+                   static_cast<unsigned>(q.s) * p.v.ld};
+  }
+  __device__ __forceinline__ void cell(const Pend& q, int i, bool fresh, float4* out) const {
+    const PhaseArgs& p = jobs[q.job];
+    if (i < p.a.B) *out = coop_cell(p.a, Ops{p.v, p.a.B}, q, i, fresh);
+  }
+};
+
 // One work unit of the persistent kernels: two vertices of degree <= 64
-// (a half-warp each; un.y = -1 when there is only one) or one vertex of
-// degree <= 128 (the whole warp, un.y = kUnitWarp).  wtab: the warp's
-// shared-memory tables.
+// (a half-warp each; un.y = -1 when there is only one) or one vertex
+// (the whole warp, un.y = kUnitWarp).  wtab: the warp's shared-memory
+// tables.  In precision 3 the proposals go to `pl`, as job `job`.
 template <class Ops>
 __device__ __forceinline__ void unit_vertices(const NodalArgs& a, const Ops& ops, int2 un, uint32_t itr, int* wtab,
-                                              CtaTally* tl, int lane, unsigned long long* my_bytes) {
+                                              CtaTally* tl, int lane, unsigned long long* my_bytes, PendList* pl,
+                                              int job) {
+  int* list = wtab + 3 * kHCap;
   if (un.y == kUnitWarp) {
-    group_vertex(a, ops, un.x, itr, wtab, wtab + kHCap, wtab + 2 * kHCap, wtab + 3 * kHCap, tl, Grp<32>(lane),
-                 my_bytes);
+    group_vertex(a, ops, un.x, itr, wtab, list, tl, Grp<32>(lane), my_bytes, nullptr, pl, job);
   } else {
     const int h = lane >> 4;
     const int vv = h ? un.y : un.x;
     if (vv >= 0)
-      group_vertex(a, ops, vv, itr, wtab + h * (kHCap / 2), wtab + kHCap + h * (kHCap / 2),
-                   wtab + 2 * kHCap + h * (kHCap / 2), wtab + 3 * kHCap + h * (kHubDegree / 2), tl, Grp<16>(lane),
-                   my_bytes);
+      group_vertex(a, ops, vv, itr, wtab + h * (3 * kHCap / 2), list + h * kPairDegree, tl, Grp<16>(lane), my_bytes,
+                   nullptr, pl, job);
   }
+  __syncwarp();
+}
+
+// item x of the two tables of `cells` cells each
+__device__ __forceinline__ void ref32_table_cell(unsigned x, unsigned cells, int B, int ld, const int* M, const int* Mt,
+                                                 const int32_t* din, const int32_t* dout, float* Trow, float* Tcol) {
+  const bool col = x >= cells;
+  const unsigned c = col ? x - cells : x;
+  const unsigned b = c / ld, i = c - b * ld;
+  float t = 0.0f;
+  if (i < static_cast<unsigned>(B)) {
+    const int m = __ldcg((col ? Mt : M) + c);
+    t = ref_term_nz(m, __int2float_rn(__ldcg((col ? dout : din) + i)), __int2float_rn(__ldcg((col ? din : dout) + b)));
+  }
+  __stcg((col ? Tcol : Trow) + c, t);
 }
 
 // Precision mode 3: the reference's old-state dS terms of every tile cell
@@ -1770,19 +2444,9 @@ __device__ __forceinline__ void unit_vertices(const NodalArgs& a, const Ops& ops
 // in the reference's float arithmetic (ref_term), 0 for empty cells.
 __device__ __forceinline__ void ref32_tables_pass(int B, int ld, const int* M, const int* Mt, const int32_t* din,
                                                   const int32_t* dout, float* Trow, float* Tcol) {
-  const long long cells = static_cast<long long>(B) * ld;
-  for (long long c = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; c < cells;
-       c += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int b = static_cast<int>(c / ld), i = static_cast<int>(c - static_cast<long long>(b) * ld);
-    float tr = 0.0f, tc = 0.0f;
-    if (i < B) {
-      const int x = __ldcg(M + c), y = __ldcg(Mt + c);
-      if (x) tr = ref_term(x, static_cast<long long>(__ldcg(din + i)) * __ldcg(dout + b));
-      if (y) tc = ref_term(y, static_cast<long long>(__ldcg(dout + i)) * __ldcg(din + b));
-    }
-    __stcg(Trow + c, tr);
-    __stcg(Tcol + c, tc);
-  }
+  const unsigned cells = static_cast<unsigned>(B) * ld;   // (the tables serve B <= 16384)
+  for (unsigned x = blockIdx.x * blockDim.x + threadIdx.x; x < 2 * cells; x += gridDim.x * blockDim.x)
+    ref32_table_cell(x, cells, B, ld, M, Mt, din, dout, Trow, Tcol);
 }
 
 template <int P, bool kSnap>
@@ -1794,22 +2458,26 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_phase(PhaseArgs p) {
   __shared__ unsigned s_ovf;
   __shared__ int2 s_own[kOwnCap];
   __shared__ int s_nown;
+  __shared__ PendList s_pl;
+  __shared__ SlotCounts s_sc;
   using Ops = DenseOpsT<LdCG, P, std::conditional_t<kSnap, LdPlain, LdCG>>;
   NodalCtl* ctl = p.a.ctl;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int gw = blockIdx.x * kPWarps + wib;
   const int nw = gridDim.x * kPWarps;
   int* wtab = dyn + wib * kPWarpInts;
-  int* htab = dyn + kPWarps * kPWarpInts;   // hub table during proposals, delta tables during apply
+  int* htab = dyn + kPWarps * kPWarpInts;   // hub region: hub tables and staging during proposals, delta tables during apply
+  int* hubtab = htab + 3 * kPhaseHubSlots;  // its second half: a hub's table
   // kSnap (B <= kSnapMaxB): the proposals read M, Mt, the chunk sums and the
   // block degrees from a copy in shared memory, taken at every batch start;
   // it shares the hub table's region (a hub's table then needs at most
-  // kSnapOff slots per array)
-  int* sM = htab + kSnapOff;
-  int* sMt = htab + kPHubSlots + kSnapOff;
-  int* sCS = htab + 2 * kPHubSlots + kSnapOff;
-  int* sdin = sCS + kSnapMaxB;
-  int* sdout = sdin + kSnapMaxB;
+  // kSnapSlots slots per array)
+  int* sM = htab + 3 * kSnapSlots;
+  int* sMt = sM + p.a.B * p.v.ld;
+  int* sCS = sMt + p.a.B * p.v.ld;
+  int* sdin = sCS + p.a.B;
+  int* sdout = sdin + p.a.B;
+  const int snap_ints = 3 * kSnapSlots + 2 * p.a.B * p.v.ld + ((3 * p.a.B + 3) & ~3);   // a multiple of 4
   DenseView vs = p.v;
   if (kSnap) {
     vs.M = sM;
@@ -1831,6 +2499,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_phase(PhaseArgs p) {
   unsigned target = 0;
   unsigned long long my_bytes = 0;
   bool converged = false;
+  if constexpr (P == 3) ref_tab_fill();   // (grid barriers lie before its first use)
   for (int sw = 0; sw < p.maxitr; sw++) {
     // data term of S for this sweep (the entropy kernel's sum)
     {
@@ -1893,31 +2562,57 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_phase(PhaseArgs p) {
         s_tally.nown = &s_nown;
         s_tally.own_cap = kOwnCap;
         s_nown = 0;
+        s_pl.n = 0;
       }
       __syncthreads();
-      const int hub_lo = __ldg(p.batch_hub + bi), hub_hi = __ldg(p.batch_hub + bi + 1);
+      const int hub_lo = __ldg(p.batch_hub + bi);
+      const int hub_hi = P == 3 && p.a.hub_units ? hub_lo : __ldg(p.batch_hub + bi + 1);   // proposed by CTAs
       const int hcta = min(hub_hi - hub_lo, static_cast<int>(gridDim.x));
-      for (int h = hub_lo + blockIdx.x; h < hub_hi; h += gridDim.x)
-        hub_vertex<Ops, kPThreads>(a, ops, __ldg(p.hubs + h), itr, htab, kPHubSlots, &sh, &my_bytes);
       // work units: two vertices of degree <= 64 (a half-warp each) or one
-      // of degree <= 128 (a warp)
+      // vertex (a warp)
       const int u_lo = __ldg(p.unit_ptr + bi), nun = __ldg(p.unit_ptr + bi + 1) - u_lo;
+      const int extra = P == 3 && p.a.hub_units ? __ldg(p.batch_hub + bi + 1) - hub_lo : 0;   // hubs as units
       const int first = (gridDim.x - hcta) * kPWarps;   // units handed out without the counter
-      if (static_cast<int>(blockIdx.x) >= hcta) {
-        // one unit per CTA in turn: a small batch then has a warp on every
-        // SM instead of 24 on a few (N = 5000, 1250 vertices a batch: 37 us a
-        // batch at B = 151 against 66 us packed)
-        const int i = wib * (gridDim.x - hcta) + (blockIdx.x - hcta);
-        if (i < nun) unit_vertices(a, ops, __ldg(p.units + u_lo + i), itr, wtab, &s_tally, lane, &my_bytes);
-      }
-      // the rest in rounds of one unit per warp, kPWarps per counter step
-      for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) s_base = first + static_cast<int>(atomicAdd(&ctl->vnext, static_cast<unsigned>(kPWarps)));
-        __syncthreads();
-        const int i0 = s_base;
-        if (i0 >= nun) break;
-        if (i0 + wib < nun) unit_vertices(a, ops, __ldg(p.units + u_lo + i0 + wib), itr, wtab, &s_tally, lane, &my_bytes);
+      // waves of proposals: the CTA's hubs, one each; then one unit per warp,
+      // dealt in turn to the CTAs without a hub; then, where units are left,
+      // kPWarps per step of a counter
+      int h = hub_lo + blockIdx.x;
+      for (bool dealt = false;;) {
+        int taken = 0;   // ints at the end of the hub region that hold a hub's table
+        if (h < hub_hi) {
+          hub_vertex<Ops, kPThreads>(a, ops, __ldg(p.hubs + h), itr, kSnap ? htab : hubtab,
+                                     kSnap ? kSnapSlots : kPhaseHubSlots, &sh, &my_bytes, nullptr, &s_pl, 0);
+          if (P == 3 && !kSnap && s_pl.p[0].cap <= kPhaseHubSlots) taken = 3 * s_pl.p[0].cap;
+          h += gridDim.x;
+        } else {
+          int i = nun + extra;
+          if (!dealt) {
+            dealt = true;
+            if (static_cast<int>(blockIdx.x) >= hcta) i = wib * (gridDim.x - hcta) + (blockIdx.x - hcta);
+          } else {
+            if (first >= nun + extra) break;
+            __syncthreads();
+            if (threadIdx.x == 0) s_base = first + static_cast<int>(atomicAdd(&ctl->vnext, static_cast<unsigned>(kPWarps)));
+            __syncthreads();
+            if (s_base >= nun + extra) break;
+            i = s_base + wib;
+          }
+          if (i < nun + extra) {
+            const int2 un = i < nun ? __ldg(p.units + u_lo + i) : make_int2(__ldg(p.hubs + hub_lo + i - nun), kUnitWarp);
+            unit_vertices(a, ops, un, itr, wtab, &s_tally, lane, &my_bytes, &s_pl, 0);
+          }
+        }
+        if constexpr (P == 3) {   // the float dS of the wave's proposals
+          __syncthreads();
+          const SingleJob<Ops> job{a, ops};
+          float* stage = reinterpret_cast<float*>(htab + (kSnap ? snap_ints : 0));
+          const int room = 3 * kPHubSlots - (kSnap ? snap_ints : 0) - taken;
+          const auto close = [&](const Pend& q, float f) { close_vertex<Ops>(a, q, f, &s_tally, &my_bytes); };
+          if (!kSnap && a.sparse) coop_eval_sparse<kPThreads>(s_pl, stage, room, &s_sc, job, close);
+          else coop_eval<kPThreads>(s_pl, stage, room, job, close);
+          __syncthreads();
+          if (threadIdx.x == 0) s_pl.n = 0;
+        }
       }
       __syncthreads();
       if (threadIdx.x == 0) tally_flush(&s_tally, ctl);
@@ -2079,6 +2774,8 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_gang(const PhaseArgs* __
   __shared__ unsigned s_ovf;
   __shared__ int2 s_own[kOwnCap];   // {v, job << 16 | chunk} of the CTA's accepted work-unit moves
   __shared__ int s_nown;
+  __shared__ PendList s_pl, s_pls;   // proposals on full tiles, on sparse tiles
+  __shared__ SlotCounts s_sc;
   unsigned ovf_seen = 0;
   using Ops = DenseOpsT<LdCG, P>;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -2086,6 +2783,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_gang(const PhaseArgs* __
   const int nw = gridDim.x * kPWarps;
   int* wtab = dyn + wib * kPWarpInts;
   int* htab = dyn + kPWarps * kPWarpInts;
+  int* hubtab = htab + 3 * kPhaseHubSlots;
   const DeltaTables dt{htab, htab + kPHubSlots, htab + 2 * kPHubSlots, htab + 2 * kPHubSlots + kPHubSlots / 2,
                        kPHubLg, kPHubLg - 1};
   unsigned target = 0;
@@ -2103,6 +2801,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_gang(const PhaseArgs* __
     s_nb[threadIdx.x] = (p.n + p.bs - 1) / p.bs;
     s_fin[threadIdx.x] = 0;
   }
+  if constexpr (P == 3) ref_tab_fill();
   __syncthreads();
 
   for (;;) {
@@ -2162,7 +2861,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_gang(const PhaseArgs* __
       // proposes
       {
         long long cells = 0;
-        if (mine && jobs[threadIdx.x].a.Trow) cells = static_cast<long long>(jobs[threadIdx.x].a.B) * jobs[threadIdx.x].a.tld;
+        if (mine && jobs[threadIdx.x].a.Trow) cells = 2ll * jobs[threadIdx.x].a.B * jobs[threadIdx.x].a.tld;
         job_prefix(cells, s_tmp, s_cp);
       }
       const long long total = s_cp[K];
@@ -2171,17 +2870,8 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_gang(const PhaseArgs* __
              c += static_cast<long long>(gridDim.x) * kPThreads) {
           const int j = find_job(s_cp, K, c);
           const PhaseArgs& p = jobs[j];
-          const long long cc = c - s_cp[j];
-          const int ld = p.a.tld, B = p.a.B;
-          const int b = static_cast<int>(cc / ld), i = static_cast<int>(cc - static_cast<long long>(b) * ld);
-          float tr = 0.0f, tc = 0.0f;
-          if (i < B) {
-            const int x = __ldcg(p.v.M + cc), y = __ldcg(p.v.Mt + cc);
-            if (x) tr = ref_term(x, static_cast<long long>(__ldcg(p.din + i)) * __ldcg(p.dout + b));
-            if (y) tc = ref_term(y, static_cast<long long>(__ldcg(p.dout + i)) * __ldcg(p.din + b));
-          }
-          __stcg(p.a.Trow + cc, tr);
-          __stcg(p.a.Tcol + cc, tc);
+          ref32_table_cell(static_cast<unsigned>(c - s_cp[j]), static_cast<unsigned>(p.a.B) * p.a.tld, p.a.B, p.a.tld,
+                           p.v.M, p.v.Mt, p.din, p.dout, p.a.Trow, p.a.Tcol);
         }
         if (grid_barrier(gc, &target, false, &s_state) < 0) return;
       }
@@ -2194,7 +2884,10 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_gang(const PhaseArgs* __
       s_tally[threadIdx.x].own_cap = kOwnCap;
       s_tally[threadIdx.x].own_tag = threadIdx.x << 16;
     }
-    if (threadIdx.x == 0) s_nown = 0;
+    if (threadIdx.x == 0) {
+      s_nown = 0;
+      s_pl.n = s_pls.n = 0;
+    }
     {
       long long nh = 0, nu = 0;
       if (mine) {
@@ -2202,39 +2895,66 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_gang(const PhaseArgs* __
         const int b = s_bi[threadIdx.x];
         nh = __ldg(p.batch_hub + b + 1) - __ldg(p.batch_hub + b);
         nu = __ldg(p.unit_ptr + b + 1) - __ldg(p.unit_ptr + b);
+        if (P == 3 && p.a.hub_units) {   // its hubs follow its units
+          nu += nh;
+          nh = 0;
+        }
       }
       job_prefix(nh, s_tmp, s_hp);
       job_prefix(nu, s_tmp, s_up);
     }
     const int H = static_cast<int>(s_hp[K]);
     const int U = static_cast<int>(s_up[K]);
-    for (int h = blockIdx.x; h < H; h += gridDim.x) {
-      const int j = find_job(s_hp, K, h);
-      const PhaseArgs& p = jobs[j];
-      const int v = __ldg(p.hubs + __ldg(p.batch_hub + s_bi[j]) + (h - static_cast<int>(s_hp[j])));
-      hub_vertex<Ops, kPThreads>(p.a, Ops{p.v, p.a.B}, v, static_cast<uint32_t>(s_sw[j]), htab, kPHubSlots, &sh,
-                                 &unused_bytes);
-    }
-    auto run_unit = [&](int u) {
-      const int j = find_job(s_up, K, u);
-      const PhaseArgs& p = jobs[j];
-      const int2 un = __ldg(p.units + __ldg(p.unit_ptr + s_bi[j]) + (u - static_cast<int>(s_up[j])));
-      unit_vertices(p.a, Ops{p.v, p.a.B}, un, static_cast<uint32_t>(s_sw[j]), wtab, &s_tally[j], lane,
-                    &unused_bytes);
-    };
     const int hcta = min(H, static_cast<int>(gridDim.x));
     const int first = (gridDim.x - hcta) * kPWarps;
-    if (static_cast<int>(blockIdx.x) >= hcta) {
-      const int i = (blockIdx.x - hcta) * kPWarps + wib;
-      if (i < U) run_unit(i);
-    }
-    for (;;) {
-      __syncthreads();
-      if (threadIdx.x == 0) s_base = first + static_cast<int>(atomicAdd(&gc->vnext, static_cast<unsigned>(kPWarps)));
-      __syncthreads();
-      const int i0 = s_base;
-      if (i0 >= U) break;
-      if (i0 + wib < U) run_unit(i0 + wib);
+    int h = blockIdx.x;
+    for (bool dealt = false;;) {   // waves as in k_nodal_phase
+      int taken = 0;
+      if (h < H) {
+        const int j = find_job(s_hp, K, h);
+        const PhaseArgs& p = jobs[j];
+        const int v = __ldg(p.hubs + __ldg(p.batch_hub + s_bi[j]) + (h - static_cast<int>(s_hp[j])));
+        PendList* pl = p.a.sparse ? &s_pls : &s_pl;
+        hub_vertex<Ops, kPThreads>(p.a, Ops{p.v, p.a.B}, v, static_cast<uint32_t>(s_sw[j]), hubtab, kPhaseHubSlots, &sh,
+                                   &unused_bytes, nullptr, pl, j);
+        if (P == 3 && pl->p[0].cap <= kPhaseHubSlots) taken = 3 * pl->p[0].cap;
+        h += gridDim.x;
+      } else {
+        int u = U;
+        if (!dealt) {
+          dealt = true;
+          if (static_cast<int>(blockIdx.x) >= hcta) u = (blockIdx.x - hcta) * kPWarps + wib;
+        } else {
+          if (first >= U) break;
+          __syncthreads();
+          if (threadIdx.x == 0) s_base = first + static_cast<int>(atomicAdd(&gc->vnext, static_cast<unsigned>(kPWarps)));
+          __syncthreads();
+          if (s_base >= U) break;
+          u = s_base + wib;
+        }
+        if (u < U) {
+          const int j = find_job(s_up, K, u);
+          const PhaseArgs& p = jobs[j];
+          const int u0 = __ldg(p.unit_ptr + s_bi[j]), nun = __ldg(p.unit_ptr + s_bi[j] + 1) - u0;
+          const int i = u - static_cast<int>(s_up[j]);
+          const int2 un = i < nun ? __ldg(p.units + u0 + i)
+                                  : make_int2(__ldg(p.hubs + __ldg(p.batch_hub + s_bi[j]) + i - nun), kUnitWarp);
+          unit_vertices(p.a, Ops{p.v, p.a.B}, un, static_cast<uint32_t>(s_sw[j]), wtab, &s_tally[j], lane,
+                        &unused_bytes, p.a.sparse ? &s_pls : &s_pl, j);
+        }
+      }
+      if constexpr (P == 3) {
+        __syncthreads();
+        float* stage = reinterpret_cast<float*>(htab);
+        const GangJobs<Ops> gj{jobs};
+        const auto close = [&](const Pend& q, float f) {
+          close_vertex<Ops>(jobs[q.job].a, q, f, &s_tally[q.job], &unused_bytes);
+        };
+        coop_eval<kPThreads>(s_pl, stage, 3 * kPHubSlots - taken, gj, close);
+        coop_eval_sparse<kPThreads>(s_pls, stage, 3 * kPHubSlots - taken, &s_sc, gj, close);
+        __syncthreads();
+        if (threadIdx.x == 0) s_pl.n = s_pls.n = 0;
+      }
     }
     __syncthreads();
     if (threadIdx.x < K && s_act[threadIdx.x]) tally_flush(&s_tally[threadIdx.x], jobs[threadIdx.x].a.ctl);
@@ -2407,6 +3127,17 @@ int nodal_phase_grid(int device) {
   if (device < 0 || device >= 64) return 0;
   nodal_configure(device);
   return g_phase_grid[device];
+}
+
+// The line: per 64 blocks packing costs what it saves when about a fifth of
+// the cells are filled (coop; batches of N = 20000 at B = 1227, e = 0.2 cells:
+// 91 us packed, 87 us whole; N = 50000 at B = 1526, 0.33: 385 against 294 us;
+// N = 4999 at B = 625, 0.2: 26 against 33 us).  A single warp also saves the
+// additions that every lane repeats: until two edges a cell (N = 50000, B =
+// 763, 1.3: 230 us packed, 259 us whole).
+bool float_ds_sparse(int64_t e, int32_t B, bool coop) {
+  const int64_t cells = static_cast<int64_t>(B) * B;
+  return B > kSnapMaxB && (coop ? 5 * e < cells : e < 2 * cells);
 }
 
 int nodal_phase_warps() { return kPWarps; }
