@@ -81,8 +81,8 @@ typedef struct usap_params {
   int32_t trace_kinds; /* trace events to emit: bit k-1 for kind k; 0 = all kinds */
   int32_t sweep_graphs;/* 1: record each stage's nodal sweep as a CUDA graph and replay it */
   int32_t persistent;  /* 1 (default): run each stage's nodal phase as one cooperative kernel
-                          when the tile is dense and B <= 4096; 0: one launch per batch.
-                          usap_batch_partition always uses per-batch launches. */
+                          when the tile is dense; 0: one launch per batch (the batched and
+                          served forms always use the cooperative kernel there). */
   int32_t persistent_ctas; /* CTAs of the cooperative kernel (one per SM); 0 = every SM */
   int32_t precision;   /* 3 (default): the reference's float nodal dS, below.
                           0: every dS term in FP64, rounded to Q32 and summed exactly.
@@ -254,10 +254,10 @@ usap_status usap_ctx_test_barrier_timeout(usap_ctx* ctx, int32_t hold_cta, int64
 /* One job solves graphs[graph] with its own Philox seed (several jobs on the
  * same graph are independent chains).  Graphs are loaded once and shared.
  * Jobs run concurrently, each on its own stream driven by one of `workers`
- * host threads (0 = automatic: 64); their kernels overlap on the GPU, and
- * their dense nodal phases (B <= 4096) run together in cooperative "gang"
- * launches that advance every waiting job by one batch a round.  Every
- * job's result equals the result of solving it alone with the same seed. */
+ * host threads (0 = automatic; at most 8 solve at a time); their nodal phases
+ * run side by side, each as one cooperative launch on a share of the SMs that
+ * follows its batch size, and their other work overlaps.  Every job's result
+ * equals the result of solving it alone with the same seed. */
 typedef struct usap_batch_job {
   int32_t graph;        /* index into graphs[] */
   uint64_t seed;        /* Philox seed of this chain */
@@ -271,9 +271,9 @@ typedef struct usap_batch_stats {
   double ms_load;       /* loading the graphs */
   int32_t workers;
   int64_t kernel_launches;
-  int64_t gang_launches;  /* cooperative launches that ran several jobs' nodal phases */
-  int64_t gang_phases;    /* job nodal phases (or resumed parts of them) in those launches */
-  double ms_gang;         /* wall time of those launches */
+  int64_t gang_launches;  /* cooperative launches of the jobs' nodal phases */
+  int64_t gang_phases;    /* nodal phases run in them (one each) */
+  double ms_gang;         /* summed wall time of those launches */
 } usap_batch_stats;
 
 usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, const usap_params* p,
@@ -329,19 +329,19 @@ usap_status usap_op_nodal_batch_prec(usap_ctx* ctx, int32_t* part, int32_t B, in
 /* --- served form: a partition service on one GPU --------------------------
  * The reference has no service; this replaces a caller running Graph_P
  * objects on its own threads.  usap_server_submit copies the edge list and
- * returns a ticket at once; worker threads (each with its own streams and
- * solver state) take requests in arrival order whenever a worker is free
+ * returns a ticket at once; worker threads take requests in arrival order
+ * whenever a worker and a solver state are free (up to 8 solve at a time)
  * and the request's device-memory footprint fits in what running requests
  * leave of the budget, so requests that arrive while others run start as
  * soon as a slot and memory free up and their kernels overlap on the GPU.
  * out_assign must stay valid until the request is taken with poll or
  * wait.  A request's result is the same as usap_partition's for the same
- * graph and parameters (the cooperative nodal kernel is not used, since it
- * would hold every SM). */
+ * graph and parameters.  As in the batched form, the requests' nodal phases
+ * run side by side on shares of the SMs. */
 typedef struct usap_server usap_server;
 typedef struct usap_server_config {
   int32_t device;
-  int32_t workers;        /* concurrent requests (0: min(32, 2 x host threads)) */
+  int32_t workers;        /* worker threads (0: min(32, 2 x host threads)); at most 8 solve at a time */
   int64_t memory_budget;  /* bytes of device memory for admitted requests (0: 80% of free) */
   int32_t reserved[4];
 } usap_server_config;

@@ -270,6 +270,8 @@ usap_status usap_ctx_test_barrier_timeout(usap_ctx* ctx, int32_t hold_cta, int64
   });
 }
 
+constexpr int kBatchWorkers = 64;
+
 usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, const usap_params* p,
                                  usap_batch_job* jobs, int32_t njobs, int32_t workers,
                                  int32_t device, usap_batch_stats* stats) {
@@ -284,12 +286,10 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
     auto t0 = std::chrono::steady_clock::now();
     int hw = static_cast<int>(std::thread::hardware_concurrency());
     if (hw <= 0) hw = 8;
-    // dense nodal phases of the concurrent solves run together in gang
-    // launches; solves mostly wait there, so more of them than host threads
-    std::unique_ptr<usap::NodalGang> gang;
+    // the solves' nodal phases share the SMs
     USAP_CUDA(cudaSetDevice(device));
-    if (usap::nodal_gang_grid(device) > 0) gang = std::make_unique<usap::NodalGang>(device);
-    int W = workers > 0 ? workers : (gang ? usap::kGangMax : std::min(32, 2 * hw));
+    usap::SmPool pool(device);
+    int W = workers > 0 ? workers : kBatchWorkers;
     W = std::max(1, std::min(W, std::max(njobs, ngraphs)));
     // load every graph once, in parallel
     std::vector<std::shared_ptr<usap::GraphResident>> res(ngraphs);
@@ -323,7 +323,7 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
     {
       int64_t want = 0;
       const int64_t dmax = usap::effective_dense_max(base);
-      for (int32_t k = 0; k < std::min<int32_t>(W, njobs); k++) {
+      for (int32_t k = 0; k < std::min<int32_t>(std::min(W, usap::kSolveSlots), njobs); k++) {
         const usap::HostGraph& hg = res[jobs[order[k]].graph]->hg;
         // initial blocks: one per vertex, or about N/7 from the SCC pass
         const int64_t b0 = base.init_mode == 1 ? hg.n : std::max<int64_t>(1, hg.n / 4);
@@ -334,7 +334,7 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
     std::atomic<int32_t> next{0};
     std::atomic<long long> launches{0};
     std::vector<std::thread> th;
-    for (int w = 0; w < std::min(W, std::max<int32_t>(njobs, 1)); w++)
+    for (int w = 0; w < std::min(std::min(W, usap::kSolveSlots), std::max<int32_t>(njobs, 1)); w++)
       th.emplace_back([&] {
         const auto lc0 = usap::launch_count();
         std::unique_ptr<usap::Job> job;
@@ -349,16 +349,10 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
             bj.status = USAP_ERR_CUDA;
             continue;
           }
-          struct GangSeat {   // counts this solve as in progress for the gang
-            usap::NodalGang* g;
-            explicit GangSeat(usap::NodalGang* gg) : g(gg) { if (g) g->enter(); }
-            ~GangSeat() { if (g) g->leave(); }
-          } seat(gang.get());
           try {
-            job->set_gang(gang.get());
+            job->set_pool(&pool);
             job->attach(res[bj.graph]);
             usap_params prm = base;
-            prm.persistent = 0;   // concurrent jobs: per-batch launches interleave
             prm.seed = bj.seed;
             job->partition(prm, bj.out_assign, &bj.result);
             bj.status = USAP_OK;
@@ -378,9 +372,9 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
       stats->ms_load = std::chrono::duration<double, std::milli>(t1 - t0).count();
       stats->workers = W;
       stats->kernel_launches = launches.load();
-      stats->gang_launches = gang ? gang->launches() : 0;
-      stats->gang_phases = gang ? gang->phases() : 0;
-      stats->ms_gang = gang ? gang->ms() : 0.0;
+      stats->gang_launches = pool.launches();
+      stats->gang_phases = pool.launches();
+      stats->ms_gang = pool.ms();
     }
     for (int32_t j = 0; j < njobs; j++)
       if (jobs[j].status != USAP_OK) throw usap::Error(jobs[j].status, "a batch job failed");

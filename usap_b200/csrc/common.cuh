@@ -288,24 +288,22 @@ __device__ __forceinline__ void ref_tab_fill() {
 
 // ref_logf of a quotient x / prod with 1 <= x, prod < 2^48 (a normal, finite,
 // positive float), without branches: the same operations on the same values
-// as ref_logf, so that several evaluations interleave.  Any other input
-// gives a value that the caller discards (the table index is in range for
-// every bit pattern).
+// as ref_logf, so that several evaluations interleave.  0 gives a finite
+// value; the table index is in range for every bit pattern.
 __device__ __forceinline__ float ref_logf_quot(float x) {
   const unsigned u = __float_as_uint(x);
   // e = exponent of x, one more where the fraction is at least sqrt(2)'s
-  // (0x3504F4); d = (m - 1) 2^23 with m = x / 2^e, negative when m < 1
+  // (0x3504F4); mb = bits of m = x / 2^e
   const int e = static_cast<int>(u - 0x3f3504f4u) >> 23;
   const unsigned mb = u - (static_cast<unsigned>(e) << 23);
-  const int d = static_cast<int>(mb - 0x3f800000u);
-  // k = 128 (m - 1) rounded half up: d / 2^16, or d / 2^17 below one, where
-  // a unit of d is half as large
-  const int k = ((d >> (15 - (d >> 31))) + 1) >> 1;
+  // k = 128 (m - 1) rounded half up = floor(floor(256 m) / 2 - 127.5), the
+  // inner floor by a downward rounding to integers above 2^23
+  const int f = static_cast<int>(__float_as_uint(__fmaf_rd(__uint_as_float(mb), 256.0f, 12582912.0f)) - 0x4b400000u);
+  const int k = (f - 255) >> 1;
   const double m = __hiloint2double(static_cast<int>((mb >> 3) + (896u << 20)), static_cast<int>(mb << 29));
   const double2 t = ref_tab()[kRefLogK0 + k];
   const double w = __fma_rn(m, t.x, -1.0);   // exact, as m * t.x is
-  double q = -1.0 / 8.0;
-  q = __fma_rn(q, w, 1.0 / 7.0);
+  double q = __fma_rn(-1.0 / 8.0, w, 1.0 / 7.0);
   q = __fma_rn(q, w, -1.0 / 6.0);
   q = __fma_rn(q, w, 1.0 / 5.0);
   q = __fma_rn(q, w, -1.0 / 4.0);
@@ -319,14 +317,18 @@ __device__ __forceinline__ float ref_logf_quot(float x) {
   return __double2float_rn(__dadd_rn(hi, l1p));
 }
 
-// ref_term(x, da * db) where x != 0, else 0, without branches (x >= 0).  The
+// the degrees' factor of a term: as a float, at least 1 (see ref_term_nz)
+__device__ __forceinline__ float ref_factor(int d) { return fmaxf(__int2float_rn(d), 1.0f); }
+
+// ref_term(x, da * db) where x != 0, else +-0, without branches (x >= 0).  The
 // degrees come as floats: they are below 2^24, so exact, and the float
 // product of two of them is the reference's long product rounded to float.
-// Where x > 0 neither degree is zero: both count x among their edges.
+// Where x > 0 neither degree is zero (both count x among their edges), so
+// degrees of at least 1 (ref_factor) change no term and keep the term of an
+// empty cell at 0 * a finite log; a chain may add +-0 (it never holds -0).
 __device__ __forceinline__ float ref_term_nz(int x, float da, float db) {
   const float xf = __int2float_rn(x);
-  const float t = __fmul_rn(xf, ref_logf_quot(quot_rn(xf, __fmul_rn(da, db))));
-  return x ? t : 0.0f;
+  return __fmul_rn(xf, ref_logf_quot(quot_rn(xf, __fmul_rn(da, db))));
 }
 
 // one term of the reference's dS: count * log((float)count / (float)prod),

@@ -169,7 +169,6 @@ struct NodalCtl {
   unsigned long long bar;   // arrivals (low 32 bits), convergence (bits 32-47) and move-list overflow (bits 48-63) arrivals
   int bar_err;
   unsigned int vnext;
-  int gang_batch;           // gang launches: next batch of the current sweep (0: a new sweep starts)
   F32Tally f32;             // precision mode 1: FP32 decisions against the FP64 values
   unsigned long long apply_scans;   // persistent kernel: batches applied by scanning all chunks (a CTA's move list overflowed)
 };
@@ -269,20 +268,15 @@ struct PhaseArgs {
   int bar_hold;             // failure injection: this CTA never arrives at a barrier (-1: none)
 };
 
-// Control block of a gang launch (several jobs' nodal phases at once).
-constexpr int kGangMax = 64;
-struct GangCtl {
-  unsigned long long bar;   // grid barrier arrivals
-  int bar_err;
-  unsigned int vnext;       // work units handed out by the counter
-  int finished[kGangMax];   // 1: the job's nodal phase is complete; 0: resume it in a later launch
-};
-
 // --- launchers (kernels_*.cu) -------------------------------------------------
 void launch_dense_build(const GraphDev& g, const int32_t* part, int B, int ld, int* M, int* Mt,
                         cudaStream_t st);
 void launch_degrees(const GraphDev& g, const int32_t* part, int B, int32_t* dout, int32_t* din,
                     cudaStream_t st);
+// copies a few words to pinned host memory by a kernel's stores: a device to
+// host copy would wait for its stream in a copy engine's queue, and hold up
+// the other streams' copies behind it for as long
+void launch_copy_out(void* host, const void* dev, size_t bytes, cudaStream_t st);
 void launch_log_pairs(const double* L, float2* T, int64_t n, cudaStream_t st);
 void launch_entropy_dense(const GraphDev& g, DenseView v, int B, const int32_t* dout,
                           const int32_t* din, unsigned long long* acc, cudaStream_t st);
@@ -310,15 +304,9 @@ int nodal_phase_grid(int device);
 // before it evaluates terms (a tile of B x B cells, `e` edges)
 bool float_ds_sparse(int64_t e, int32_t B, bool coop);
 int nodal_phase_warps();   // warps of one of its CTAs
-int nodal_gang_grid(int device);
 // largest B whose hub tables fit the persistent kernel's shared memory
 int nodal_phase_max_blocks();
 void launch_nodal_phase(const PhaseArgs& p, int grid, cudaStream_t st);
-// nodal phases of K <= kGangMax jobs (PhaseArgs array in device memory)
-// (the launch ends once fewer than exit_below jobs are unfinished)
-// (prec: every job's precision mode)
-void launch_nodal_gang(const PhaseArgs* jobs_dev, int K, GangCtl* gc, int exit_below, int grid, int prec,
-                       cudaStream_t st);
 void launch_nodal_propose_dense(const NodalArgs& a, DenseView v, const HubList& hubs,
                                 const StreamPair& sp);
 void launch_nodal_propose_sorted(const NodalArgs& a, SortedView v, const HubList& hubs,

@@ -165,10 +165,10 @@ Job::~Job() {
   if (st_) cudaStreamDestroy(st_);
 }
 
-// waits for the job's stream; with blocking waits the host thread sleeps
-// instead of spinning, so many concurrent jobs can share the host cores
-void Job::wait() {
-  if (blocking_wait_) {
+// waits for the job's stream; a blocking wait sleeps instead of spinning, so
+// that the host threads of many concurrent solves can share the cores
+void Job::wait(bool block) {
+  if (block) {
     USAP_CUDA(cudaEventRecord(ev_wait_, st_));
     USAP_CUDA(cudaEventSynchronize(ev_wait_));
   } else {
@@ -596,7 +596,7 @@ int32_t Job::merge_apply(int32_t* part, int32_t B, int32_t btm) {
   launch_merge_union(B, sidx_alt_, best_s_, btm, union_work_, root_, merged_dev_, st_);
   launch_merge_relabel(hg_->n, B, part, root_, present_, newlabel_, cub_tmp_, cub_bytes_, st_);
   int32_t merged = 0;
-  USAP_CUDA(cudaMemcpyAsync(&h_ctl_->itr, merged_dev_, sizeof(int32_t), cudaMemcpyDeviceToHost, st_));
+  launch_copy_out(&h_ctl_->itr, merged_dev_, sizeof(int32_t), st_);
   wait();
   merged = h_ctl_->itr;
   return merged;
@@ -696,7 +696,7 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
   const int32_t n = hg_->n;
   const int32_t nb = (n + bs_ - 1) / bs_;
   // a vertex per warp while a batch fits the grid's warps that way, else two
-  const bool single = !gang_ && bs_ <= static_cast<int64_t>(grid) * nodal_phase_warps();
+  const bool single = bs_ <= static_cast<int64_t>(grid) * nodal_phase_warps();
   if (batch_hub_bs_ != bs_ || units_single_ != single) {   // first hub of each batch, for this batch size
     const std::vector<int32_t>& hub_ids = gr_->hub_ids;
     std::vector<int32_t> bh(static_cast<size_t>(nb) + 1);
@@ -794,10 +794,9 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
     // neighbours a CTA is faster than a warp
     pa.a.hub_units = !pa.a.shadow && B <= 768 && g_.maxk < 65536 && g_.maxdeg <= 2048;
   }
-  // precision mode 3: the old-state term tables of the persistent kernels,
-  // single-job and gang (one pass over the tile and a grid barrier per
-  // batch), where the proposals' own evaluation costs more: see kRefTabMin
-  if (pa.a.coop && !pa.a.sparse && (gang_ || static_cast<int64_t>(bs_) * B > kRefTabMin * grid)) {
+  // precision mode 3: the old-state term tables (one pass over the tile and a
+  // grid barrier per batch), where the proposals' own evaluation costs more: see kRefTabMin
+  if (pa.a.coop && !pa.a.sparse && static_cast<int64_t>(bs_) * B > kRefTabMin * grid) {
     const size_t cells = static_cast<size_t>(ld_) * ld_;
     if (cells > tcap_) {
       dfree(Trow_);
@@ -809,12 +808,6 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
     pa.a.Trow = Trow_;
     pa.a.Tcol = Tcol_;
     pa.a.tld = ld_;
-  }
-  if (gang_ && !timed) {
-    gang_->run(pa, st_);
-    USAP_CUDA(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(NodalCtl), cudaMemcpyDeviceToHost, st_));
-    wait();
-    return 0.0f;
   }
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (timed) {
@@ -829,8 +822,8 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
   }
   launch_nodal_phase(pa, grid, st_);
   if (timed) USAP_CUDA(cudaEventRecord(e1, st_));
-  USAP_CUDA(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(NodalCtl), cudaMemcpyDeviceToHost, st_));
-  wait();
+  launch_copy_out(h_ctl_, ctl_, sizeof(NodalCtl), st_);
+  wait(pool_ != nullptr);   // milliseconds, beside other solves' phases
   if (h_ctl_->bar_err) throw Error(USAP_ERR_INTERNAL, "persistent nodal kernel: a grid barrier timed out");
   float ms = 0;
   if (timed) USAP_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -911,6 +904,37 @@ void Job::emit_trace(int kind, int stage, int itr, int beg, int32_t B, const int
 }
 
 // --- the whole solve ------------------------------------------------------------
+namespace {
+
+struct PoolSeat {   // the solve is in progress
+  SmPool* p;
+  int64_t batch;
+  PoolSeat(SmPool* pool, int64_t b) : p(pool), batch(b) {
+    if (p) p->enter(batch);
+  }
+  ~PoolSeat() {
+    if (p) p->leave(batch);
+  }
+  PoolSeat(const PoolSeat&) = delete;
+  PoolSeat& operator=(const PoolSeat&) = delete;
+};
+
+struct PoolCtas {   // CTAs of one nodal phase: from the pool, or all
+  SmPool* p;
+  int n;
+  std::chrono::steady_clock::time_point t0;
+  PoolCtas(SmPool* pool, int64_t batch, int most) : p(pool), n(pool ? pool->acquire(batch, most) : most) {
+    t0 = std::chrono::steady_clock::now();
+  }
+  ~PoolCtas() {
+    if (p) p->release(n, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
+  }
+  PoolCtas(const PoolCtas&) = delete;
+  PoolCtas& operator=(const PoolCtas&) = delete;
+};
+
+}  // namespace
+
 void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res, const int32_t* init) {
   if (!loaded()) throw Error(USAP_ERR_STATE, "no graph loaded");
   USAP_CUDA(cudaSetDevice(device_));
@@ -930,6 +954,7 @@ void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res,
   const int32_t maxitr = p.max_num_nodal_itr;
   bs_ = n / p.num_batch_nodal_update;
   if (bs_ < 1) bs_ = 1;
+  const PoolSeat seat(pool_, bs_);
   const int stats = p.stats ? 1 : 0;
   const bool use_graphs = p.sweep_graphs != 0 && !stats;
   trace_mask_ = p.trace_kinds ? p.trace_kinds : 7;
@@ -1004,12 +1029,11 @@ void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res,
     const double model_d = model_S(n, hg_->e, B);
     trace_prev_moves_ = 0;
     const bool phase_ok = dense && !use_graphs && maxitr > 0 && B <= nodal_phase_max_blocks() && !trace_on(2);
-    // the gang's delta-table keys pack (job, cell) into 31 bits: B <= 4096
-    const bool in_gang = gang_ != nullptr && phase_ok && !stats && B <= 4096;
-    const int pgrid = phase_ok && (p.persistent || in_gang) ? nodal_phase_grid(device_) : 0;
-    const int pctas = p.persistent_ctas > 0 ? std::min(pgrid, static_cast<int>(p.persistent_ctas)) : pgrid;
+    const int pgrid = phase_ok && (p.persistent || pool_) ? nodal_phase_grid(device_) : 0;
+    const int pmost = p.persistent_ctas > 0 ? std::min(pgrid, static_cast<int>(p.persistent_ctas)) : pgrid;
     if (pgrid > 0) {
-      const float ms = nodal_phase(part, B, stage, seed, W, thr, model_d, maxitr, stats, pctas, stats != 0);
+      const PoolCtas ctas(pool_, bs_, pmost);
+      const float ms = nodal_phase(part, B, stage, seed, W, thr, model_d, maxitr, stats, ctas.n, stats != 0);
       d2h += sizeof(NodalCtl);
       if (stats) {
         res->ms_nodal_kernel += ms;
@@ -1036,7 +1060,7 @@ void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res,
       auto launch_one = [&] {
         if (exec) USAP_CUDA(cudaGraphLaunch(exec, st_));
         else enqueue_sweep(part, B, dense, stage, seed, W, thr, model_d, stats);
-        USAP_CUDA(cudaMemcpyAsync(h_ring_ + (launched & 1), ctl_, sizeof(NodalCtl), cudaMemcpyDeviceToHost, st_));
+        launch_copy_out(h_ring_ + (launched & 1), ctl_, sizeof(NodalCtl), st_);
         USAP_CUDA(cudaEventRecord(ev_sweep_[launched & 1], st_));
         launched++;
         d2h += sizeof(NodalCtl);
@@ -1085,7 +1109,7 @@ void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res,
                                     (static_cast<long long>(hg_->in_ptr[end]) - hg_->in_ptr[beg]);
             const CtlArgs ca{1, W, thr, model_d, ide_q_, ide_n_, end - beg, edges};
             nodal_batch(part, B, dense, beg, end, stage, seed, beg == 0, stats, ca);
-            USAP_CUDA(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(NodalCtl), cudaMemcpyDeviceToHost, st_));
+            launch_copy_out(h_ctl_, ctl_, sizeof(NodalCtl), st_);
             wait();
             NodalCtl c = *h_ctl_;
             emit_trace(2, stage, itr, beg, B, part, dense, c.S_q, c.S_ninf, static_cast<long long>(c.cum_q),
@@ -1094,7 +1118,7 @@ void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res,
             if (c.done) break;
           }
         }
-        USAP_CUDA(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(NodalCtl), cudaMemcpyDeviceToHost, st_));
+        launch_copy_out(h_ctl_, ctl_, sizeof(NodalCtl), st_);
         wait();
         d2h += sizeof(NodalCtl);
         if (stats) {
@@ -1131,7 +1155,7 @@ void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res,
     if (pgrid <= 0) {
       if (!dense) sb_.build(g_, part, B, false, true, st_);
       entropy_launch(part, B, dense);
-      USAP_CUDA(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(NodalCtl), cudaMemcpyDeviceToHost, st_));
+      launch_copy_out(h_ctl_, ctl_, sizeof(NodalCtl), st_);
       wait();
       data_fin = -static_cast<long long>(h_ctl_->entropy_acc);
       d2h += sizeof(NodalCtl);
@@ -1329,7 +1353,7 @@ int64_t Job::op_entropy(const int32_t* part, int32_t B, int32_t dense_max) {
   const bool dense = B <= dense_max;
   prepare_nodal_blocks(slots_[0], B, dense);
   entropy_launch(slots_[0], B, dense);
-  USAP_CUDA(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(NodalCtl), cudaMemcpyDeviceToHost, st_));
+  launch_copy_out(h_ctl_, ctl_, sizeof(NodalCtl), st_);
   USAP_CUDA(cudaStreamSynchronize(st_));
   return add_sat(q32_host(model_S(hg_->n, hg_->e, B)), -static_cast<long long>(h_ctl_->entropy_acc));
 }
@@ -1401,7 +1425,7 @@ void Job::op_nodal_batch(int32_t* part, int32_t B, int32_t dense_max, int32_t be
   if (prop_q) USAP_CUDA(cudaMemcpyAsync(prop_q, rp_q_, sizeof(int64_t) * cnt, cudaMemcpyDeviceToHost, st_));
   if (prop_ninf) USAP_CUDA(cudaMemcpyAsync(prop_ninf, rp_n_, sizeof(int32_t) * cnt, cudaMemcpyDeviceToHost, st_));
   if (prec_ && prop_f) USAP_CUDA(cudaMemcpyAsync(prop_f, rp_f_, sizeof(double) * cnt, cudaMemcpyDeviceToHost, st_));
-  USAP_CUDA(cudaMemcpyAsync(h_ctl_, ctl_, sizeof(NodalCtl), cudaMemcpyDeviceToHost, st_));
+  launch_copy_out(h_ctl_, ctl_, sizeof(NodalCtl), st_);
   USAP_CUDA(cudaStreamSynchronize(st_));
   prec_ = 0;
   if (cum_q) *cum_q = static_cast<int64_t>(h_ctl_->cum_q);

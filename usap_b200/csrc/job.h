@@ -150,51 +150,35 @@ struct GraphResident {
 // parse_tsv_device; `in` is then ignored)
 std::shared_ptr<GraphResident> load_graph(int device, const usap_graph& in, HostGraph* pre = nullptr);
 
-// Runs the dense nodal phases of concurrent solves together in single
-// cooperative launches (k_nodal_gang); see gang.cpp.
-class NodalGang {
+// Solves in progress at a time in the batched and served forms.  The streams
+// of a context share its (by default 8) hardware queues, and a kernel behind
+// another solve's running nodal phase in a queue waits for milliseconds: with
+// 16 solves a merge phase took 6 ms on average, with 8 0.14 ms.  Eight nodal
+// phases fill the SMs.
+constexpr int kSolveSlots = 8;
+
+// The SMs that concurrent solves' nodal phases share (smpool.cpp).
+class SmPool {
  public:
-  explicit NodalGang(int device);
-  ~NodalGang();
-  NodalGang(const NodalGang&) = delete;
-  NodalGang& operator=(const NodalGang&) = delete;
-  // a solve starts / ends: a launch waits for every solve in progress to
-  // reach its nodal phase (or for kGangWait)
-  void enter();
-  void leave();
-  // runs this nodal phase in the next gang launch, after the work queued on
-  // job_stream; returns when it is done
-  void run(const PhaseArgs& pa, cudaStream_t job_stream);
+  explicit SmPool(int device);
+  // a solve with batches of `batch` vertices starts / ends
+  void enter(int64_t batch);
+  void leave(int64_t batch);
+  // CTAs for its next nodal phase, at most `most` (waits for them), given back
+  // with the phase's duration
+  int acquire(int64_t batch, int most);
+  void release(int ctas, double ms);
   long long launches() const { return launches_; }
-  long long phases() const { return jobs_run_; }
   double ms() const { return ms_; }
 
  private:
-  struct Pending {
-    PhaseArgs pa;
-    cudaEvent_t ready = nullptr;
-    std::chrono::steady_clock::time_point since;
-    bool done = false;
-    bool waited = false;
-    std::string error;
-  };
-  bool ready_to_launch() const;
-  void launch(const std::vector<Pending*>& batch);
-  int device_;
-  int grid_ = 0;
   std::mutex mu_;
   std::condition_variable cv_;
-  std::vector<Pending*> pending_;
-  int live_ = 0;
-  bool busy_ = false;
-  cudaStream_t st_ = nullptr;
-  PhaseArgs* h_jobs_ = nullptr;
-  PhaseArgs* d_jobs_ = nullptr;
-  GangCtl* h_ctl_ = nullptr;
-  GangCtl* d_ctl_ = nullptr;
-  long long launches_ = 0, jobs_run_ = 0;
+  int total_, free_;
+  int64_t live_ = 0;                     // batch vertices of the solves in progress
+  uint64_t next_ = 0, serving_ = 0;      // phases are admitted in arrival order
+  long long launches_ = 0;
   double ms_ = 0.0;
-  std::chrono::steady_clock::time_point last_end_{};
 };
 
 class Job {
@@ -216,9 +200,8 @@ class Job {
   }
   const std::shared_ptr<GraphResident>& graph() const { return gr_; }
   // host threads sleep (instead of spinning) while waiting for the device
-  void set_blocking_wait(bool on) { blocking_wait_ = on; }
-  // dense nodal phases go to this gang instead of a launch of their own
-  void set_gang(NodalGang* g) { gang_ = g; }
+  // nodal phases run on SMs of this pool, beside other solves' phases
+  void set_pool(SmPool* p) { pool_ = p; }
   void set_trace(usap_trace_fn fn, void* user) {
     trace_ = fn;
     trace_user_ = user;
@@ -301,9 +284,8 @@ class Job {
   cudaEvent_t ev_wait_ = nullptr;
   cudaEvent_t ev_sweep_[2] = {nullptr, nullptr};   // sweep done + control copied
   NodalCtl* h_ring_ = nullptr;                     // pinned, two control copies
-  bool blocking_wait_ = false;
-  NodalGang* gang_ = nullptr;
-  void wait();
+  SmPool* pool_ = nullptr;
+  void wait(bool block = false);
   std::shared_ptr<GraphResident> gr_;
   const HostGraph* hg_ = nullptr;
   GraphDev g_;                       // the graph's arrays + this job's hub scratch

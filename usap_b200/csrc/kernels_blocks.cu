@@ -189,7 +189,17 @@ __global__ void k_log_pairs(int64_t n, const double* __restrict__ L, float2* __r
   }
 }
 
+__global__ void k_copy_out(int* __restrict__ host, const int* __restrict__ dev, int n) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) host[i] = __ldcg(dev + i);
+}
+
 }  // namespace
+
+void launch_copy_out(void* host, const void* dev, size_t bytes, cudaStream_t st) {
+  k_copy_out<<<1, 64, 0, st>>>(static_cast<int*>(host), static_cast<const int*>(dev),
+                               static_cast<int>(bytes / sizeof(int)));
+  USAP_LAUNCHED();
+}
 
 void launch_log_pairs(const double* L, float2* T, int64_t n, cudaStream_t st) {
   if (n <= 0) return;

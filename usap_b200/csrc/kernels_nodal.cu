@@ -38,8 +38,8 @@
 // evaluates their float dS together.
 // State written inside that kernel (the partition, M, degrees, chunk sums,
 // moves) is otherwise read through L2 (ld.cg); the non-coherent path is
-// used only for data that no phase writes.  The gang kernel runs the same
-// phase for many jobs at once.
+// used only for data that no phase writes.  The phases
+// of concurrent solves run side by side, each on fewer CTAs.
 #include <cmath>
 #include <mutex>
 #include <type_traits>
@@ -518,7 +518,7 @@ constexpr int kNbr16 = 2;   // 4 bytes a block: out, in
 // A proposal: v moves from block r to s.  In precision 3 it lies in shared
 // memory until its float dS is evaluated.
 struct __align__(16) Pend {
-  int mode, job;   // kNbr*; the gang's job
+  int mode;        // kNbr*
   bool hub;        // its chunks are not listed
   const int* tab;  // v's neighbour-block weights (kNbr8, kNbr16), or the hash's keys
   const int *two, *twi;   // the hash's out- and in-weights
@@ -560,8 +560,9 @@ __device__ __forceinline__ void nbr_weights(const Pend& q, int i, int* wo, int* 
 }
 
 __device__ __forceinline__ void set_factors(Pend& q) {
-  q.fo = make_float4(q.dr_out, q.ds_out, q.dr_in, q.ds_in);
-  q.fn = make_float4(q.dr_out - q.kout, q.ds_out + q.kout, q.dr_in - q.kin, q.ds_in + q.kin);
+  q.fo = make_float4(ref_factor(q.dr_out), ref_factor(q.ds_out), ref_factor(q.dr_in), ref_factor(q.ds_in));
+  q.fn = make_float4(ref_factor(q.dr_out - q.kout), ref_factor(q.ds_out + q.kout), ref_factor(q.dr_in - q.kin),
+                     ref_factor(q.ds_in + q.kin));
 }
 
 // the four new 2x2 terms (subtracted, in this order)
@@ -638,7 +639,7 @@ __device__ __noinline__ float ref32_nodal(const Ops ops, const int32_t* __restri
     oload(g.gl);
     for (int base = 0; base < B; base += G) {
       const int R = nR, S = nS, Rc = nRc, Sc = nSc;
-      const float di = __int2float_rn(ndi), dn = __int2float_rn(ndn);
+      const float di = ref_factor(ndi), dn = ref_factor(ndn);
       oload(base + G + g.gl);
       if (!__any_sync(0xffffffffu, (R | S | Rc | Sc) != 0)) continue;
       const float t0 = ref_term_nz(R, di, dor);
@@ -664,7 +665,7 @@ __device__ __noinline__ float ref32_nodal(const Ops ops, const int32_t* __restri
   nload(g.gl);
   for (int base = 0; base < B; base += G) {
     int R = nR, S = nS, Rc = nRc, Sc = nSc;
-    const float di = __int2float_rn(ndi), dn = __int2float_rn(ndn);
+    const float di = ref_factor(ndi), dn = ref_factor(ndn);
     nload(base + G + g.gl);
     const int i = base + g.gl;
     // v's edges towards block i are part of M[r,i] (out) and M[i,r] (in)
@@ -748,7 +749,7 @@ __device__ __forceinline__ float ref32_sparse_pass(float dS, const Ops& ops, con
     if (lane < n) e = queue[head + lane];
     const int j = e.y >> 24;
     const float fa = (j & 1) ? ff.y : ff.x, fb = (j & 1) ? ff.w : ff.z;
-    dS = ref32_run(dS, ref_term_nz(e.x, __int2float_rn(e.y & 0xffffff), (j & 2) ? fb : fa), kNew, buf, lane);
+    dS = ref32_run(dS, ref_term_nz(e.x, ref_factor(e.y & 0xffffff), (j & 2) ? fb : fa), kNew, buf, lane);
   };
   load(2 * lane);
   for (int base = 0; base < B; base += 64) {
@@ -870,13 +871,12 @@ struct CtaTally {
   unsigned long long cum, moves, near;
   int ninf;
   F32Tally f32;
-  // persistent kernels: the edge chunks {v, own_tag | chunk} of the CTA's
-  // accepted moves, so that its apply pass visits only those (null
-  // elsewhere); *nown, shared by the CTA's tallies, counts past own_cap when
-  // the list overflows; own_tag is the job index << 16 in the gang kernel
+  // persistent kernel: the edge chunks {v, chunk} of the CTA's accepted
+  // moves, so that its apply pass visits only those (null elsewhere); *nown
+  // counts past own_cap when the list overflows
   int2* own;
   int* nown;
-  int own_cap, own_tag;
+  int own_cap;
 };
 
 // the accepted dS that the convergence test sums: the exact value, or in
@@ -948,7 +948,7 @@ __device__ __forceinline__ void close_vertex(const NodalArgs& a, const Pend& q, 
     const int nch = q.deg > 32 ? (q.deg + 31) >> 5 : 1;   // the vertex's chunks (one even without edges)
     const int i0 = atomicAdd(tl->nown, nch);
     for (int c = 0; c < nch; c++)
-      if (i0 + c < tl->own_cap) tl->own[i0 + c] = make_int2(q.v, tl->own_tag | c);
+      if (i0 + c < tl->own_cap) tl->own[i0 + c] = make_int2(q.v, c);
   }
   // precision 3 also reads, for the old-state and again for the new-state
   // terms, rows r and s and columns r and s of M and both degree arrays:
@@ -965,7 +965,7 @@ __device__ __forceinline__ void close_vertex(const NodalArgs& a, const Pend& q, 
 // (hashed: 8 * G slots of key, out- and in-weight); list: KN * G ints.  With
 // a.hub_units a warp also takes larger degrees, in steps of KN * G
 // neighbours.  Closes the proposal, or in precision 3 leaves it in shared
-// memory (the next entry of *pl, or *slot without a list; job: its job) for
+// memory (the next entry of *pl, or *slot without a list) for
 // its float dS to be evaluated; returns whether it did.
 template <int G>
 constexpr int kGroupNbrs = G == 32 ? kHubDegree / 32 : kPairDegree / 16;
@@ -973,7 +973,7 @@ constexpr int kGroupNbrs = G == 32 ? kHubDegree / 32 : kPairDegree / 16;
 template <class Ops, int G>
 __device__ __forceinline__ bool group_vertex(const NodalArgs& a, const Ops& ops, int v, uint32_t itr, int* tab,
                                              int* list, CtaTally* tl, const Grp<G>& g, unsigned long long* my_bytes,
-                                             Pend* slot, PendList* pl, int job) {
+                                             Pend* slot, PendList* pl) {
   using LD = typename Ops::Ld;
   using LDT = typename Ops::LdT;
   constexpr int KN = kGroupNbrs<G>;
@@ -1154,7 +1154,6 @@ __device__ __forceinline__ bool group_vertex(const NodalArgs& a, const Ops& ops,
       Pend& q = pl ? pl->p[atomicAdd(&pl->n, 1)] : *slot;
       q.mode = mode;
       q.hub = false;
-      q.job = job;
       q.tab = key;
       q.two = two;
       q.twi = twi;
@@ -1221,7 +1220,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_nodal_propose(NodalArgs a, Ops 
   for (int v = a.beg + blockIdx.x * kWarps + wib; v < a.end; v += nwarps) {
     int* const tab = s_tab[wib];
     const bool live = group_vertex(a, ops, v, itr, tab, s_list[wib], &s_tally, Grp<32>(lane), &my_bytes,
-                                   Ops::kP == 3 ? s_pend + wib : nullptr, nullptr, 0);
+                                   Ops::kP == 3 ? s_pend + wib : nullptr, nullptr);
     if constexpr (Ops::kP == 3) {
       if (live) {   // warp-uniform
         const float f = ref32_eval(a, ops, s_pend[wib], tab, tab + kHCap, tab + 2 * kHCap,
@@ -1252,12 +1251,12 @@ struct HubShared {
 // region; with a list, precision 3, the arrays follow one another from the
 // region's end); each thread loads four neighbours at once, and up to four
 // occupied slots at once for the terms.  In precision 3 the proposal is left
-// in pl's first entry (as job `job`), or, without a list, warp 0 evaluates
+// in pl's first entry, or, without a list, warp 0 evaluates
 // its float dS (chain: kQueueInts ints).
 template <class Ops, int NT>
 __device__ __forceinline__ void hub_vertex(const NodalArgs& a, const Ops& ops, int v, uint32_t itr, int* stab,
                                            int scap, HubShared<NT / 32>* sh, unsigned long long* my_bytes,
-                                           int* chain, PendList* pl, int job) {
+                                           int* chain, PendList* pl) {
   using LD = typename Ops::Ld;
   using LDT = typename Ops::LdT;
   constexpr int NW = NT / 32;
@@ -1410,7 +1409,6 @@ __device__ __forceinline__ void hub_vertex(const NodalArgs& a, const Ops& ops, i
       if (lane == 0) {
         q.mode = kNbrHash;
         q.hub = true;
-        q.job = job;
         q.tab = key;
         q.two = two;
         q.twi = twi;
@@ -1473,7 +1471,7 @@ __global__ void __launch_bounds__(kHubThreads) k_nodal_propose_hub(NodalArgs a, 
     __syncthreads();
   }
   for (int h = hub_lo + blockIdx.x; h < hub_hi; h += gridDim.x)
-    hub_vertex<Ops, kHubThreads>(a, ops, __ldg(hubs + h), itr, dyn, smem_cap, &sh, &my_bytes, s_chain, nullptr, 0);
+    hub_vertex<Ops, kHubThreads>(a, ops, __ldg(hubs + h), itr, dyn, smem_cap, &sh, &my_bytes, s_chain, nullptr);
   if (a.stats && threadIdx.x == 0 && my_bytes) atomicAdd(&a.ctl->bytes, my_bytes);
 }
 
@@ -1734,7 +1732,6 @@ constexpr int kDeltaHashed = 0, kDeltaGlobal = 1, kDeltaDense = 2;
 struct DeltaTables {
   int *mkey, *mval, *ckey, *cval;
   int mlg, clg;   // capacities 1 << mlg, 1 << clg
-  int tag = 0;    // job number << 24 when the tables serve several jobs
   int mode = kDeltaHashed;
   int dB = 0;     // kDeltaDense: B
 };
@@ -1760,7 +1757,7 @@ __device__ __forceinline__ bool table_add(int* key, int* val, int lg, int k, int
 }
 
 __device__ __forceinline__ void cs_add(const DeltaTables& t, int* CS, int key, int d) {
-  if (!table_add(t.ckey, t.cval, t.clg, t.tag | key, d)) atomicAdd(CS + key, d);
+  if (!table_add(t.ckey, t.cval, t.clg, key, d)) atomicAdd(CS + key, d);
 }
 
 __device__ __forceinline__ void tile_add(const DeltaTables& t, int* M, int* Mt, int* CS, int ld, int cld, int x,
@@ -1778,7 +1775,7 @@ __device__ __forceinline__ void tile_add(const DeltaTables& t, int* M, int* Mt, 
     atomicAdd(CS + y * cld + x / kChunk, d);
     return;
   }
-  if (table_add(t.mkey, t.mval, t.mlg, t.tag | (x * ld + y), d)) return;
+  if (table_add(t.mkey, t.mval, t.mlg, x * ld + y, d)) return;
   atomicAdd(M + static_cast<long long>(x) * ld + y, d);
   atomicAdd(Mt + static_cast<long long>(y) * ld + x, d);
   cs_add(t, CS, x * cld + y / kChunk, d);
@@ -2107,19 +2104,19 @@ __device__ __forceinline__ unsigned long long apply_bytes(const NodalArgs& a, in
 template <class Ops>
 __device__ __forceinline__ float4 coop_cell(const NodalArgs& a, const Ops& ops, const Pend& q, int i, bool fresh) {
   using LDT = typename Ops::LdT;
-  const bool rs = i == q.r || i == q.s;
-  if (!fresh && a.Trow) {
-    const long long ro = static_cast<long long>(q.r) * a.tld + i, so = static_cast<long long>(q.s) * a.tld + i;
+  const int r = q.r, s = q.s;
+  const bool rs = i == r || i == s;
+  const unsigned ro = static_cast<unsigned>(r) * ops.v.ld + i, so = static_cast<unsigned>(s) * ops.v.ld + i;
+  if (!fresh && a.Trow)
     return make_float4(__ldcg(a.Trow + ro), __ldcg(a.Trow + so), rs ? 0.0f : __ldcg(a.Tcol + ro),
                        rs ? 0.0f : __ldcg(a.Tcol + so));
-  }
   if (fresh && rs) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  int R = ops.get(q.r, i), S = ops.get(q.s, i), Rc = 0, Sc = 0;
+  int R = LDT::ld(ops.v.M + ro), S = LDT::ld(ops.v.M + so), Rc = 0, Sc = 0;
   if (!rs) {   // columns skip i in {r, s}
-    Rc = ops.get_t(q.r, i);
-    Sc = ops.get_t(q.s, i);
+    Rc = LDT::ld(ops.v.Mt + ro);
+    Sc = LDT::ld(ops.v.Mt + so);
   }
-  const float di = __int2float_rn(LDT::ld(a.din + i)), dn = __int2float_rn(LDT::ld(a.dout + i));
+  const float di = ref_factor(LDT::ld(a.din + i)), dn = ref_factor(LDT::ld(a.dout + i));
   const float4 f = fresh ? q.fn : q.fo;
   if (fresh) {   // v's edges towards block i are part of M[r,i] (out) and M[i,r] (in)
     int wo, wi;
@@ -2134,9 +2131,10 @@ __device__ __forceinline__ float4 coop_cell(const NodalArgs& a, const Ops& ops, 
 }
 
 // The float dS of the listed proposals, handed to close(q, f) by one thread
-// each (CTA-collective).  stage: `room` floats; job: SingleJob or GangJobs.
-template <int NT, class JobFn, class CloseFn>
-__device__ __forceinline__ void coop_eval(const PendList& pl, float* stage, int room, JobFn job, CloseFn close) {
+// each (CTA-collective).  stage: `room` floats.
+template <int NT, class Ops, class CloseFn>
+__device__ __forceinline__ void coop_eval(const NodalArgs& a, const Ops& ops, const PendList& pl, float* stage,
+                                          int room, CloseFn close) {
   constexpr int NW = NT / 32;
   const int np = pl.n;
   if (np == 0) return;
@@ -2145,24 +2143,18 @@ __device__ __forceinline__ void coop_eval(const PendList& pl, float* stage, int 
   const int nprod = NT - 32 * nc;        // threads that evaluate
   const bool adds = wib >= NW - nc;
   const int mine = (wib - (NW - nc)) * 32 + lane;
-  int bmax = 0, bmine = 0;
-  for (int k = lane; k < np; k += 32) bmax = max(bmax, job.blocks(pl.p[k].job));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
-  // chunks of CB blocks, equal shares of the largest B: at most about four
+  // chunks of CB blocks, equal shares of B: at most about four
   // cells per evaluating thread, so that the last chunk's additions, which
   // overlap nothing, stay short, and both buffers within the room.  (A row of
   // the staging area is an odd number of 16-byte words: no bank conflicts
   // among the adding lanes.)
   const int most = max(8, min(4 * nprod / np, (room / (8 * np) - 1) & ~1));
-  const int nch = (bmax + most - 1) / most;
-  const int CB = ((bmax + nch - 1) / nch + 1) & ~1, stride = 4 * CB + 4;
+  const int B = a.B, nch = (B + most - 1) / most;
+  const int CB = ((B + nch - 1) / nch + 1) & ~1, stride = 4 * CB + 4;
   float dS = 0.0f, c0 = 0.0f, c1 = 0.0f, c2 = 0.0f, c3 = 0.0f;
   const bool has = adds && mine < np;
-  if (has) {
-    bmine = job.blocks(pl.p[mine].job);
-    corner_terms(pl.p[mine], &c0, &c1, &c2, &c3);   // due between the passes
-  }
+  if (has) corner_terms(pl.p[mine], &c0, &c1, &c2, &c3);   // due between the passes
+  const int ks = threadIdx.x / CB, os = threadIdx.x - ks * CB;
   const int dk = nprod / CB, dr = nprod - dk * CB;   // from one of a thread's cells to its next
   for (int t = 0; t <= 2 * nch; t++) {
     if (!adds) {
@@ -2170,9 +2162,10 @@ __device__ __forceinline__ void coop_eval(const PendList& pl, float* stage, int 
         const bool fresh = t >= nch;
         const int b0 = (fresh ? t - nch : t) * CB;
         float* st = stage + (t & 1) * np * stride;
-        int k = threadIdx.x / CB, o = threadIdx.x - k * CB;
-        for (; k < np;) {
-          job.cell(pl.p[k], b0 + o, fresh, reinterpret_cast<float4*>(st + k * stride + 4 * o));
+        int k = ks, o = os;
+        while (k < np) {
+          if (b0 + o < B)
+            *reinterpret_cast<float4*>(st + k * stride + 4 * o) = coop_cell(a, ops, pl.p[k], b0 + o, fresh);
           k += dk;
           o += dr;
           if (o >= CB) {
@@ -2184,7 +2177,7 @@ __device__ __forceinline__ void coop_eval(const PendList& pl, float* stage, int 
     } else if (has && t > 0) {
       const bool fresh = t > nch;
       const int b0 = (fresh ? t - 1 - nch : t - 1) * CB;
-      const int n = min(CB, bmine - b0);
+      const int n = min(CB, B - b0);
       const float4* st = reinterpret_cast<const float4*>(stage + ((t - 1) & 1) * np * stride + mine * stride);
       if (!fresh) {
 #pragma unroll 8
@@ -2220,15 +2213,9 @@ struct SlotCounts {
   int n[2][kMaxSlots];
 };
 
-// a tile, the offsets of rows r and s in it, and the block degrees
-struct RowPtrs {
-  const int *M, *Mt, *din, *dout;
-  unsigned r, s;
-};
-
-template <int NT, class JobFn, class CloseFn>
-__device__ __forceinline__ void coop_eval_sparse(const PendList& pl, float* stage, int room, SlotCounts* sc, JobFn job,
-                                                 CloseFn close) {
+template <int NT, class Ops, class CloseFn>
+__device__ __forceinline__ void coop_eval_sparse(const NodalArgs& a, const Ops& ops, const PendList& pl, float* stage,
+                                                 int room, SlotCounts* sc, CloseFn close) {
   constexpr int NW = NT / 32;
   const int np = pl.n;
   if (np == 0) return;
@@ -2237,11 +2224,7 @@ __device__ __forceinline__ void coop_eval_sparse(const PendList& pl, float* stag
   const int pw = NW - nc;
   const bool adds = wib >= pw;
   const int mine = (wib - pw) * 32 + lane;
-  int bmax = 0;
-  for (int k = lane; k < np; k += 32) bmax = max(bmax, job.blocks(pl.p[k].job));
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, o));
-  const int nch = (bmax + 63) >> 6;
+  const int B = a.B, nch = (B + 63) >> 6;
   // m chunks of every proposal per step, in two sets of np * m slots
   const int m = min(nch, max(1, min(kMaxSlots, room / (2 * kSlot)) / np));
   const int nst = (nch + m - 1) / m, per = np * m;
@@ -2257,15 +2240,15 @@ __device__ __forceinline__ void coop_eval_sparse(const PendList& pl, float* stag
     if (t >= 2 * nst) return;
     const Pend& q = pl.p[k];
     const int i = (((t >= nst ? t - nst : t) * m + c) << 6) + 2 * lane;
-    if (i >= job.blocks(q.job)) return;
+    if (i >= B) return;
     // (rows and degree arrays are readable up to an even number of blocks)
-    const RowPtrs rp = job.rows(q);
-    nx[0] = __ldcg(reinterpret_cast<const int2*>(rp.M + (rp.r + i)));
-    nx[1] = __ldcg(reinterpret_cast<const int2*>(rp.M + (rp.s + i)));
-    nx[2] = __ldcg(reinterpret_cast<const int2*>(rp.Mt + (rp.r + i)));
-    nx[3] = __ldcg(reinterpret_cast<const int2*>(rp.Mt + (rp.s + i)));
-    nx[4] = __ldcg(reinterpret_cast<const int2*>(rp.din + i));
-    nx[5] = __ldcg(reinterpret_cast<const int2*>(rp.dout + i));
+    const unsigned r = static_cast<unsigned>(q.r) * ops.v.ld + i, s = static_cast<unsigned>(q.s) * ops.v.ld + i;
+    nx[0] = __ldcg(reinterpret_cast<const int2*>(ops.v.M + r));
+    nx[1] = __ldcg(reinterpret_cast<const int2*>(ops.v.M + s));
+    nx[2] = __ldcg(reinterpret_cast<const int2*>(ops.v.Mt + r));
+    nx[3] = __ldcg(reinterpret_cast<const int2*>(ops.v.Mt + s));
+    nx[4] = __ldcg(reinterpret_cast<const int2*>(a.din + i));
+    nx[5] = __ldcg(reinterpret_cast<const int2*>(a.dout + i));
   };
   const unsigned lanes_below = (1u << lane) - 1u;
   const int k0 = wib % np, step_k = pw % np, c0x = wib / np, step_c = pw / np;
@@ -2338,7 +2321,7 @@ __device__ __forceinline__ void coop_eval_sparse(const PendList& pl, float* stag
             const int b0 = __shfl_sync(0xffffffffu, dn0, from), b1 = __shfl_sync(0xffffffffu, dn1, from);
             const int d = (j & 2) ? ((k & 4) ? b1 : b0) : ((k & 4) ? a1 : a0);
             const float fa = (j & 1) ? ff.y : ff.x, fb = (j & 1) ? ff.w : ff.z;
-            const float term = ref_term_nz(static_cast<int>(w & 0xffffffu), __int2float_rn(d), (j & 2) ? fb : fa);
+            const float term = ref_term_nz(static_cast<int>(w & 0xffffffu), ref_factor(d), (j & 2) ? fb : fa);
             if (e < ((total + 3) & ~3)) slot[e ^ sw] = __float_as_int(term);   // zeros up to a multiple of 4
           }
           if (lane == 0) sc->n[t & 1][x] = total;
@@ -2371,53 +2354,22 @@ __device__ __forceinline__ void coop_eval_sparse(const PendList& pl, float* stag
   if (has) close(pl.p[mine], dS);
 }
 
-// what the evaluation asks of the proposals' jobs: one job, or the gang's
-template <class Ops>
-struct SingleJob {
-  const NodalArgs& a;
-  const Ops& ops;
-  __device__ __forceinline__ int blocks(int) const { return a.B; }
-  __device__ __forceinline__ RowPtrs rows(const Pend& q) const {
-    return RowPtrs{ops.v.M, ops.v.Mt, a.din, a.dout, static_cast<unsigned>(q.r) * ops.v.ld,
-                   static_cast<unsigned>(q.s) * ops.v.ld};
-  }
-  __device__ __forceinline__ void cell(const Pend& q, int i, bool fresh, float4* out) const {
-    if (i < a.B) *out = coop_cell(a, ops, q, i, fresh);
-  }
-};
-
-template <class Ops>
-struct GangJobs {
-  const PhaseArgs* jobs;
-  __device__ __forceinline__ int blocks(int j) const { return jobs[j].a.B; }
-  __device__ __forceinline__ RowPtrs rows(const Pend& q) const {
-    const PhaseArgs& p = jobs[q.job];
-    return RowPtrs{p.v.M, p.v.Mt, p.a.din, p.a.dout, static_cast<unsigned>(q.r) * p.v.ld,
-                   static_cast<unsigned>(q.s) * p.v.ld};
-  }
-  __device__ __forceinline__ void cell(const Pend& q, int i, bool fresh, float4* out) const {
-    const PhaseArgs& p = jobs[q.job];
-    if (i < p.a.B) *out = coop_cell(p.a, Ops{p.v, p.a.B}, q, i, fresh);
-  }
-};
-
 // One work unit of the persistent kernels: two vertices of degree <= 64
 // (a half-warp each; un.y = -1 when there is only one) or one vertex
 // (the whole warp, un.y = kUnitWarp).  wtab: the warp's shared-memory
-// tables.  In precision 3 the proposals go to `pl`, as job `job`.
+// tables.  In precision 3 the proposals go to `pl`.
 template <class Ops>
 __device__ __forceinline__ void unit_vertices(const NodalArgs& a, const Ops& ops, int2 un, uint32_t itr, int* wtab,
-                                              CtaTally* tl, int lane, unsigned long long* my_bytes, PendList* pl,
-                                              int job) {
+                                              CtaTally* tl, int lane, unsigned long long* my_bytes, PendList* pl) {
   int* list = wtab + 3 * kHCap;
   if (un.y == kUnitWarp) {
-    group_vertex(a, ops, un.x, itr, wtab, list, tl, Grp<32>(lane), my_bytes, nullptr, pl, job);
+    group_vertex(a, ops, un.x, itr, wtab, list, tl, Grp<32>(lane), my_bytes, nullptr, pl);
   } else {
     const int h = lane >> 4;
     const int vv = h ? un.y : un.x;
     if (vv >= 0)
       group_vertex(a, ops, vv, itr, wtab + h * (3 * kHCap / 2), list + h * kPairDegree, tl, Grp<16>(lane), my_bytes,
-                   nullptr, pl, job);
+                   nullptr, pl);
   }
   __syncwarp();
 }
@@ -2431,7 +2383,7 @@ __device__ __forceinline__ void ref32_table_cell(unsigned x, unsigned cells, int
   float t = 0.0f;
   if (i < static_cast<unsigned>(B)) {
     const int m = __ldcg((col ? Mt : M) + c);
-    t = ref_term_nz(m, __int2float_rn(__ldcg((col ? dout : din) + i)), __int2float_rn(__ldcg((col ? din : dout) + b)));
+    t = ref_term_nz(m, ref_factor(__ldcg((col ? dout : din) + i)), ref_factor(__ldcg((col ? din : dout) + b)));
   }
   __stcg((col ? Tcol : Trow) + c, t);
 }
@@ -2492,7 +2444,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_phase(PhaseArgs p) {
   const int mode = p.a.B >= kDeltaGlobalMinB ? kDeltaGlobal
                    : (p.a.B * p.a.B <= 2 * kPHubSlots ? kDeltaDense : kDeltaHashed);
   const DeltaTables dt{htab, htab + kPHubSlots, htab + 2 * kPHubSlots, htab + 2 * kPHubSlots + kPHubSlots / 2,
-                       kPHubLg, kPHubLg - 1, 0, mode, p.a.B};
+                       kPHubLg, kPHubLg - 1, mode, p.a.B};
   const int B = p.a.B;
   unsigned ovf_seen = 0;   // overflow count at the previous proposal barrier
   const int64_t cells = static_cast<int64_t>(B) * B;
@@ -2581,7 +2533,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_phase(PhaseArgs p) {
         int taken = 0;   // ints at the end of the hub region that hold a hub's table
         if (h < hub_hi) {
           hub_vertex<Ops, kPThreads>(a, ops, __ldg(p.hubs + h), itr, kSnap ? htab : hubtab,
-                                     kSnap ? kSnapSlots : kPhaseHubSlots, &sh, &my_bytes, nullptr, &s_pl, 0);
+                                     kSnap ? kSnapSlots : kPhaseHubSlots, &sh, &my_bytes, nullptr, &s_pl);
           if (P == 3 && !kSnap && s_pl.p[0].cap <= kPhaseHubSlots) taken = 3 * s_pl.p[0].cap;
           h += gridDim.x;
         } else {
@@ -2599,17 +2551,16 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_phase(PhaseArgs p) {
           }
           if (i < nun + extra) {
             const int2 un = i < nun ? __ldg(p.units + u_lo + i) : make_int2(__ldg(p.hubs + hub_lo + i - nun), kUnitWarp);
-            unit_vertices(a, ops, un, itr, wtab, &s_tally, lane, &my_bytes, &s_pl, 0);
+            unit_vertices(a, ops, un, itr, wtab, &s_tally, lane, &my_bytes, &s_pl);
           }
         }
         if constexpr (P == 3) {   // the float dS of the wave's proposals
           __syncthreads();
-          const SingleJob<Ops> job{a, ops};
           float* stage = reinterpret_cast<float*>(htab + (kSnap ? snap_ints : 0));
           const int room = 3 * kPHubSlots - (kSnap ? snap_ints : 0) - taken;
           const auto close = [&](const Pend& q, float f) { close_vertex<Ops>(a, q, f, &s_tally, &my_bytes); };
-          if (!kSnap && a.sparse) coop_eval_sparse<kPThreads>(s_pl, stage, room, &s_sc, job, close);
-          else coop_eval<kPThreads>(s_pl, stage, room, job, close);
+          if (!kSnap && a.sparse) coop_eval_sparse<kPThreads>(a, ops, s_pl, stage, room, &s_sc, close);
+          else coop_eval<kPThreads>(a, ops, s_pl, stage, room, close);
           __syncthreads();
           if (threadIdx.x == 0) s_pl.n = 0;
         }
@@ -2688,368 +2639,6 @@ __global__ void __launch_bounds__(kPThreads, 1) k_nodal_phase(PhaseArgs p) {
   if (p.a.stats && my_bytes) atomicAdd(&ctl->bytes, my_bytes);
 }
 
-// --- gang of jobs: many nodal phases in one cooperative launch ---------------
-// first index j with pref[j + 1] > x (pref ascending, pref[0] = 0, x < pref[K])
-__device__ __forceinline__ int find_job(const long long* pref, int K, long long x) {
-  int lo = 0, hi = K;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (pref[mid] <= x) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// writes the deltas of the gang's jobs (key = job << 24 | index) to their
-// tiles (CTA-collective; tables cleared on the way)
-__device__ __forceinline__ void gang_tables_flush(const DeltaTables& t, const PhaseArgs* __restrict__ jobs) {
-  __syncthreads();
-  for (int i = threadIdx.x; i < (1 << t.mlg); i += blockDim.x) {
-    const int k = t.mkey[i];
-    if (k < 0) continue;
-    const int d = t.mval[i];
-    t.mkey[i] = -1;
-    t.mval[i] = 0;
-    if (d == 0) continue;
-    const int j = k >> 24, idx = k & 0xffffff;
-    const PhaseArgs& p = jobs[j];
-    const int ld = p.v.ld, cld = p.v.cld;
-    const int x = idx / ld, y = idx - x * ld;
-    atomicAdd(p.M + static_cast<long long>(x) * ld + y, d);
-    atomicAdd(p.Mt + static_cast<long long>(y) * ld + x, d);
-    DeltaTables tj = t;
-    tj.tag = j << 24;
-    cs_add(tj, p.CS, x * cld + y / kChunk, d);
-    cs_add(tj, p.CS, y * cld + x / kChunk, d);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < (1 << t.clg); i += blockDim.x) {
-    const int k = t.ckey[i];
-    if (k < 0) continue;
-    const int d = t.cval[i];
-    t.ckey[i] = -1;
-    t.cval[i] = 0;
-    if (d) atomicAdd(jobs[k >> 24].CS + (k & 0xffffff), d);
-  }
-  __syncthreads();
-}
-
-// out[0] = 0, out[j + 1] = v_0 + ... + v_j over the gang's jobs, where
-// thread j holds v_j (0 for j >= K); CTA-collective, K <= kGangMax = 64
-__device__ __forceinline__ void job_prefix(long long v, long long* tmp, long long* out) {
-  if (threadIdx.x < kGangMax) tmp[threadIdx.x] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int l = threadIdx.x;
-    const long long a = warp_incl_scan_ll(tmp[l], l);
-    const long long ta = __shfl_sync(0xffffffffu, a, 31);
-    const long long b = warp_incl_scan_ll(tmp[l + 32], l) + ta;
-    out[l + 1] = a;
-    out[l + 33] = b;
-    if (l == 0) out[0] = 0;
-  }
-  __syncthreads();
-}
-
-// The nodal phases of K jobs (each at some stage of its own solve, dense
-// tile, B <= 4096) in one cooperative launch.  Every round advances each
-// unfinished job by one batch: jobs that start a sweep get their entropy
-// pass and sweep-start bookkeeping first; then the proposals of all jobs'
-// current batches (hubs one per CTA, then work units) share the grid, and
-// so do their apply passes, while one thread per job closes its batch.  A
-// job leaves the gang when its convergence test fires or its sweep budget
-// is spent; the launch ends with the last job.  The arithmetic per job is
-// that of k_nodal_phase (same device functions, same order of the integer
-// sums' terms is irrelevant), so each job's result equals its solo solve.
-template <int P>
-__global__ void __launch_bounds__(kPThreads, 1) k_nodal_gang(const PhaseArgs* __restrict__ jobs, int K, GangCtl* gc,
-                                                             int exit_below) {
-  extern __shared__ __align__(16) int dyn[];
-  __shared__ CtaTally s_tally[kGangMax];
-  __shared__ HubShared<kPWarps> sh;
-  __shared__ int s_bi[kGangMax], s_sw[kGangMax], s_act[kGangMax], s_nb[kGangMax];
-  __shared__ int s_fin[kGangMax];   // finished in the last round: its final data term is due
-  __shared__ long long s_hp[kGangMax + 1], s_up[kGangMax + 1], s_cp[kGangMax + 1], s_tmp[kGangMax];
-  __shared__ int s_base, s_state;
-  __shared__ unsigned s_ovf;
-  __shared__ int2 s_own[kOwnCap];   // {v, job << 16 | chunk} of the CTA's accepted work-unit moves
-  __shared__ int s_nown;
-  __shared__ PendList s_pl, s_pls;   // proposals on full tiles, on sparse tiles
-  __shared__ SlotCounts s_sc;
-  unsigned ovf_seen = 0;
-  using Ops = DenseOpsT<LdCG, P>;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int gw = blockIdx.x * kPWarps + wib;
-  const int nw = gridDim.x * kPWarps;
-  int* wtab = dyn + wib * kPWarpInts;
-  int* htab = dyn + kPWarps * kPWarpInts;
-  int* hubtab = htab + 3 * kPhaseHubSlots;
-  const DeltaTables dt{htab, htab + kPHubSlots, htab + 2 * kPHubSlots, htab + 2 * kPHubSlots + kPHubSlots / 2,
-                       kPHubLg, kPHubLg - 1};
-  unsigned target = 0;
-  unsigned long long unused_bytes = 0;
-  // a job may resume where an earlier launch left it: at batch gang_batch
-  // of the sweep it had started (ctl->sweeps counts started sweeps)
-  if (threadIdx.x < K) {
-    const PhaseArgs& p = jobs[threadIdx.x];
-    const int gb = __ldcg(&p.a.ctl->gang_batch);
-    const int started = static_cast<int>(__ldcg(&p.a.ctl->sweeps));
-    const int done = __ldcg(&p.a.ctl->done);
-    s_bi[threadIdx.x] = gb;
-    s_sw[threadIdx.x] = gb > 0 ? started - 1 : started;
-    s_act[threadIdx.x] = !done && s_sw[threadIdx.x] < p.maxitr ? 1 : 0;
-    s_nb[threadIdx.x] = (p.n + p.bs - 1) / p.bs;
-    s_fin[threadIdx.x] = 0;
-  }
-  if constexpr (P == 3) ref_tab_fill();
-  __syncthreads();
-
-  for (;;) {
-    __syncthreads();
-    const bool mine = threadIdx.x < K && s_act[threadIdx.x];
-    const int count = __syncthreads_count(mine);
-    const int fin = __syncthreads_or(threadIdx.x < K && s_fin[threadIdx.x]);
-    // no job left, or enough are done: the rest resume in the next launch
-    const bool leaving = count == 0 || count < exit_below;
-    const int start = leaving ? 0 : __syncthreads_or(mine && s_bi[threadIdx.x] == 0);
-    if (start || fin) {
-      // data term of S: at the sweep start of the jobs that begin one, and
-      // of the final state of those that finished (read by the host)
-      {
-        long long cells = 0;
-        if ((start && mine && s_bi[threadIdx.x] == 0) || (threadIdx.x < K && s_fin[threadIdx.x])) {
-          const long long B = jobs[threadIdx.x].a.B;
-          cells = B * B;
-        }
-        job_prefix(cells, s_tmp, s_cp);
-      }
-      const long long total = s_cp[K];
-      long long acc = 0;
-      int cj = -1;
-      for (long long c = static_cast<long long>(blockIdx.x) * kPThreads + threadIdx.x; c < total;
-           c += static_cast<long long>(gridDim.x) * kPThreads) {
-        const int j = find_job(s_cp, K, c);
-        if (j != cj) {
-          if (cj >= 0 && acc) atomicAdd(&jobs[cj].a.ctl->entropy_acc, static_cast<unsigned long long>(acc));
-          acc = 0;
-          cj = j;
-        }
-        const PhaseArgs& p = jobs[j];
-        const long long cc = c - s_cp[j];
-        const int B = p.a.B;
-        const int i = static_cast<int>(cc / B), jj = static_cast<int>(cc - static_cast<long long>(i) * B);
-        const int m = __ldcg(p.v.M + static_cast<long long>(i) * p.v.ld + jj);
-        if (m) acc += q32(g_term(p.a.L, m, __ldcg(p.din + jj), __ldcg(p.dout + i)));
-      }
-      if (cj >= 0 && acc) atomicAdd(&jobs[cj].a.ctl->entropy_acc, static_cast<unsigned long long>(acc));
-      __syncthreads();
-      if (threadIdx.x < K) s_fin[threadIdx.x] = 0;
-      if (start) {
-        if (grid_barrier(gc, &target, false, &s_state) < 0) return;
-        if (blockIdx.x == 0 && threadIdx.x < K && s_act[threadIdx.x] && s_bi[threadIdx.x] == 0) {
-          const PhaseArgs& p = jobs[threadIdx.x];
-          ctl_sweep_start(p.a.ctl, p.W, p.ide_q, p.ide_n);
-          p.a.ctl->entropy_acc = 0;
-        }
-        if (grid_barrier(gc, &target, false, &s_state) < 0) return;
-      }
-    }
-    if (leaving) break;
-    if constexpr (P == 3) {
-      // precision 3: the old-state term tables of every unfinished job's
-      // batch (as the single-job kernel's ref32_tables_pass), before anyone
-      // proposes
-      {
-        long long cells = 0;
-        if (mine && jobs[threadIdx.x].a.Trow) cells = 2ll * jobs[threadIdx.x].a.B * jobs[threadIdx.x].a.tld;
-        job_prefix(cells, s_tmp, s_cp);
-      }
-      const long long total = s_cp[K];
-      if (total > 0) {
-        for (long long c = static_cast<long long>(blockIdx.x) * kPThreads + threadIdx.x; c < total;
-             c += static_cast<long long>(gridDim.x) * kPThreads) {
-          const int j = find_job(s_cp, K, c);
-          const PhaseArgs& p = jobs[j];
-          ref32_table_cell(static_cast<unsigned>(c - s_cp[j]), static_cast<unsigned>(p.a.B) * p.a.tld, p.a.B, p.a.tld,
-                           p.v.M, p.v.Mt, p.din, p.dout, p.a.Trow, p.a.Tcol);
-        }
-        if (grid_barrier(gc, &target, false, &s_state) < 0) return;
-      }
-    }
-    // proposals of every unfinished job's current batch
-    if (threadIdx.x < K) {
-      s_tally[threadIdx.x] = CtaTally{0, 0, 0, 0};
-      s_tally[threadIdx.x].own = s_own;
-      s_tally[threadIdx.x].nown = &s_nown;
-      s_tally[threadIdx.x].own_cap = kOwnCap;
-      s_tally[threadIdx.x].own_tag = threadIdx.x << 16;
-    }
-    if (threadIdx.x == 0) {
-      s_nown = 0;
-      s_pl.n = s_pls.n = 0;
-    }
-    {
-      long long nh = 0, nu = 0;
-      if (mine) {
-        const PhaseArgs& p = jobs[threadIdx.x];
-        const int b = s_bi[threadIdx.x];
-        nh = __ldg(p.batch_hub + b + 1) - __ldg(p.batch_hub + b);
-        nu = __ldg(p.unit_ptr + b + 1) - __ldg(p.unit_ptr + b);
-        if (P == 3 && p.a.hub_units) {   // its hubs follow its units
-          nu += nh;
-          nh = 0;
-        }
-      }
-      job_prefix(nh, s_tmp, s_hp);
-      job_prefix(nu, s_tmp, s_up);
-    }
-    const int H = static_cast<int>(s_hp[K]);
-    const int U = static_cast<int>(s_up[K]);
-    const int hcta = min(H, static_cast<int>(gridDim.x));
-    const int first = (gridDim.x - hcta) * kPWarps;
-    int h = blockIdx.x;
-    for (bool dealt = false;;) {   // waves as in k_nodal_phase
-      int taken = 0;
-      if (h < H) {
-        const int j = find_job(s_hp, K, h);
-        const PhaseArgs& p = jobs[j];
-        const int v = __ldg(p.hubs + __ldg(p.batch_hub + s_bi[j]) + (h - static_cast<int>(s_hp[j])));
-        PendList* pl = p.a.sparse ? &s_pls : &s_pl;
-        hub_vertex<Ops, kPThreads>(p.a, Ops{p.v, p.a.B}, v, static_cast<uint32_t>(s_sw[j]), hubtab, kPhaseHubSlots, &sh,
-                                   &unused_bytes, nullptr, pl, j);
-        if (P == 3 && pl->p[0].cap <= kPhaseHubSlots) taken = 3 * pl->p[0].cap;
-        h += gridDim.x;
-      } else {
-        int u = U;
-        if (!dealt) {
-          dealt = true;
-          if (static_cast<int>(blockIdx.x) >= hcta) u = (blockIdx.x - hcta) * kPWarps + wib;
-        } else {
-          if (first >= U) break;
-          __syncthreads();
-          if (threadIdx.x == 0) s_base = first + static_cast<int>(atomicAdd(&gc->vnext, static_cast<unsigned>(kPWarps)));
-          __syncthreads();
-          if (s_base >= U) break;
-          u = s_base + wib;
-        }
-        if (u < U) {
-          const int j = find_job(s_up, K, u);
-          const PhaseArgs& p = jobs[j];
-          const int u0 = __ldg(p.unit_ptr + s_bi[j]), nun = __ldg(p.unit_ptr + s_bi[j] + 1) - u0;
-          const int i = u - static_cast<int>(s_up[j]);
-          const int2 un = i < nun ? __ldg(p.units + u0 + i)
-                                  : make_int2(__ldg(p.hubs + __ldg(p.batch_hub + s_bi[j]) + i - nun), kUnitWarp);
-          unit_vertices(p.a, Ops{p.v, p.a.B}, un, static_cast<uint32_t>(s_sw[j]), wtab, &s_tally[j], lane,
-                        &unused_bytes, p.a.sparse ? &s_pls : &s_pl, j);
-        }
-      }
-      if constexpr (P == 3) {
-        __syncthreads();
-        float* stage = reinterpret_cast<float*>(htab);
-        const GangJobs<Ops> gj{jobs};
-        const auto close = [&](const Pend& q, float f) {
-          close_vertex<Ops>(jobs[q.job].a, q, f, &s_tally[q.job], &unused_bytes);
-        };
-        coop_eval<kPThreads>(s_pl, stage, 3 * kPHubSlots - taken, gj, close);
-        coop_eval_sparse<kPThreads>(s_pls, stage, 3 * kPHubSlots - taken, &s_sc, gj, close);
-        __syncthreads();
-        if (threadIdx.x == 0) s_pl.n = s_pls.n = 0;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x < K && s_act[threadIdx.x]) tally_flush(&s_tally[threadIdx.x], jobs[threadIdx.x].a.ctl);
-    const int nown = s_nown;
-    if (grid_barrier(gc, &target, false, &s_state, nown > kOwnCap, &s_ovf) < 0) return;
-    // as in k_nodal_phase: every CTA reads the same overflow count here
-    const bool scan_all = s_ovf != ovf_seen;
-    ovf_seen = s_ovf;
-    // apply + commit of every job's batch; one thread per job closes it.
-    // Each CTA applies the moves it accepted (its listed work-unit chunks
-    // and its moved hubs), or, after an overflow anywhere, every CTA takes
-    // its share of all jobs' batch chunks.
-    if (blockIdx.x == 0) {
-      if (threadIdx.x < K && s_act[threadIdx.x]) {
-        const PhaseArgs& p = jobs[threadIdx.x];
-        const int beg = s_bi[threadIdx.x] * p.bs, end = min(p.n, beg + p.bs);
-        const long long edges = (static_cast<long long>(__ldg(p.a.out_ptr + end)) - __ldg(p.a.out_ptr + beg)) +
-                                (static_cast<long long>(__ldg(p.a.in_ptr + end)) - __ldg(p.a.in_ptr + beg));
-        const CtlArgs ca{1, p.W, p.thr, p.model_d, p.ide_q, p.ide_n, end - beg, edges};
-        ctl_batch_end(p.a.ctl, ca);
-      }
-      if (threadIdx.x == 0) gc->vnext = 0;
-    }
-    tables_clear(dt);
-    if (scan_all) {
-      long long c = 0;
-      if (mine) {
-        const PhaseArgs& p = jobs[threadIdx.x];
-        const int beg = s_bi[threadIdx.x] * p.bs, end = min(p.n, beg + p.bs);
-        c = __ldg(p.chunk_ptr + end) - __ldg(p.chunk_ptr + beg);
-      }
-      job_prefix(c, s_tmp, s_cp);
-      const long long C = s_cp[K];
-      for (long long q = gw; q < C; q += nw) {
-        const int j = find_job(s_cp, K, q);
-        const PhaseArgs& p = jobs[j];
-        const int beg = s_bi[j] * p.bs, end = min(p.n, beg + p.bs);
-        const int2 ch = __ldg(p.g.chunks + __ldg(p.chunk_ptr + beg) + (q - s_cp[j]));
-        DeltaTables tj = dt;
-        tj.tag = j << 24;
-        apply_chunk<LdCG, LdCG>(ch, p.g, p.part, p.a.move_to, p.a.from, beg, end, tj, p.v.ld, p.M, p.Mt,
-                                p.v.cld, p.CS, p.dout, p.din, lane);
-      }
-    } else {
-      __syncthreads();
-      for (int i = wib; i < nown; i += kPWarps) {
-        const int2 e = s_own[i];
-        const int j = e.y >> 16;
-        const PhaseArgs& p = jobs[j];
-        const int beg = s_bi[j] * p.bs, end = min(p.n, beg + p.bs);
-        DeltaTables tj = dt;
-        tj.tag = j << 24;
-        apply_chunk<LdCG, LdCG>(make_int2(e.x, e.y & 0xffff), p.g, p.part, p.a.move_to, p.a.from, beg, end, tj,
-                                p.v.ld, p.M, p.Mt, p.v.cld, p.CS, p.dout, p.din, lane);
-      }
-      for (int h = blockIdx.x; h < H; h += gridDim.x) {   // the hubs this CTA proposed for
-        const int j = find_job(s_hp, K, h);
-        const PhaseArgs& p = jobs[j];
-        const int v = __ldg(p.hubs + __ldg(p.batch_hub + s_bi[j]) + (h - static_cast<int>(s_hp[j])));
-        if (__ldcg(p.a.move_to + v) < 0) continue;   // CTA-uniform
-        const int beg = s_bi[j] * p.bs, end = min(p.n, beg + p.bs);
-        DeltaTables tj = dt;
-        tj.tag = j << 24;
-        const int64_t q1 = __ldg(p.chunk_ptr + v + 1);
-        for (int64_t q = __ldg(p.chunk_ptr + v) + wib; q < q1; q += kPWarps)
-          apply_chunk<LdCG, LdCG>(__ldg(p.g.chunks + q), p.g, p.part, p.a.move_to, p.a.from, beg, end, tj, p.v.ld,
-                                  p.M, p.Mt, p.v.cld, p.CS, p.dout, p.din, lane);
-      }
-    }
-    gang_tables_flush(dt, jobs);
-    if (grid_barrier(gc, &target, false, &s_state) < 0) return;
-    // advance every job by one batch
-    if (threadIdx.x < K && s_act[threadIdx.x]) {
-      const int j = threadIdx.x;
-      const PhaseArgs& p = jobs[j];
-      const int done = *reinterpret_cast<volatile int*>(&p.a.ctl->done);
-      if (++s_bi[j] == s_nb[j]) {
-        s_bi[j] = 0;
-        s_sw[j]++;
-      }
-      if (done || s_sw[j] >= p.maxitr) {
-        s_act[j] = 0;
-        s_fin[j] = 1;
-      }
-    }
-  }
-  // where each job stands: finished, or the batch to resume at
-  __syncthreads();
-  if (blockIdx.x == 0 && threadIdx.x < K) {
-    const int j = threadIdx.x;
-    gc->finished[j] = s_act[j] ? 0 : 1;
-    jobs[j].a.ctl->gang_batch = s_act[j] ? s_bi[j] : 0;
-  }
-}
-
 // the hub CTAs run on a second stream, concurrently with the warp kernel
 template <class Ops>
 void launch_propose(const NodalArgs& a, Ops ops, const HubList& hubs, const StreamPair& sp) {
@@ -3081,7 +2670,6 @@ void launch_propose(const NodalArgs& a, Ops ops, const HubList& hubs, const Stre
 
 namespace {
 int g_phase_grid[64];
-int g_gang_grid[64];
 }
 
 // dynamic shared memory limits, set once per device, and the grid of the
@@ -3097,7 +2685,7 @@ void nodal_configure(int device) {
     USAP_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
     USAP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     // one grid for every precision mode: the fewest co-resident CTAs
-    int per_phase = 1 << 30, per_gang = 1 << 30;
+    int per_phase = 1 << 30;
     auto configure = [&](auto tag) {
       constexpr int P = decltype(tag)::value;
       USAP_CUDA(cudaFuncSetAttribute(k_nodal_propose_hub<DenseOpsT<LdNC, P>>,
@@ -3106,20 +2694,16 @@ void nodal_configure(int device) {
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       USAP_CUDA(cudaFuncSetAttribute(k_nodal_phase<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
       USAP_CUDA(cudaFuncSetAttribute(k_nodal_phase<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
-      USAP_CUDA(cudaFuncSetAttribute(k_nodal_gang<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, psmem));
-      int a = 0, a2 = 0, b = 0;
+      int a = 0, a2 = 0;
       USAP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_nodal_phase<P, false>, kPThreads, kPSmemBytes));
       USAP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a2, k_nodal_phase<P, true>, kPThreads, kPSmemBytes));
-      USAP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_nodal_gang<P>, kPThreads, kPSmemBytes));
       per_phase = std::min(per_phase, std::min(a, a2));
-      per_gang = std::min(per_gang, b);
     };
     configure(std::integral_constant<int, 0>{});
     configure(std::integral_constant<int, 1>{});
     configure(std::integral_constant<int, 2>{});
     configure(std::integral_constant<int, 3>{});
     g_phase_grid[device] = coop ? per_phase * sms : 0;
-    g_gang_grid[device] = coop ? per_gang * sms : 0;
   });
 }
 
@@ -3142,23 +2726,10 @@ bool float_ds_sparse(int64_t e, int32_t B, bool coop) {
 
 int nodal_phase_warps() { return kPWarps; }
 
-int nodal_gang_grid(int device) {
-  if (device < 0 || device >= 64) return 0;
-  nodal_configure(device);
-  return g_gang_grid[device];
-}
-
 // the apply pass keys a tile cell as x * ld + y in 31 bits
 int nodal_phase_max_blocks() { return 32768; }
 
-// the cooperative kernels of precision mode `prec` (0, 1, 2, 3)
-static const void* gang_kernel(int prec) {
-  if (prec == 1) return reinterpret_cast<const void*>(k_nodal_gang<1>);
-  if (prec == 2) return reinterpret_cast<const void*>(k_nodal_gang<2>);
-  if (prec == 3) return reinterpret_cast<const void*>(k_nodal_gang<3>);
-  return reinterpret_cast<const void*>(k_nodal_gang<0>);
-}
-
+// the cooperative kernel of precision mode `prec` (0, 1, 2, 3);
 // snap: the variant that copies the tile into shared memory (B <= kSnapMaxB)
 static const void* phase_kernel(int prec, bool snap) {
   if (snap) {
@@ -3171,18 +2742,6 @@ static const void* phase_kernel(int prec, bool snap) {
   if (prec == 2) return reinterpret_cast<const void*>(k_nodal_phase<2, false>);
   if (prec == 3) return reinterpret_cast<const void*>(k_nodal_phase<3, false>);
   return reinterpret_cast<const void*>(k_nodal_phase<0, false>);
-}
-
-void launch_nodal_gang(const PhaseArgs* jobs_dev, int K, GangCtl* gc, int exit_below, int grid, int prec,
-                       cudaStream_t st) {
-  const PhaseArgs* j = jobs_dev;
-  int k = K;
-  GangCtl* c = gc;
-  int e = exit_below;
-  void* kargs[] = {&j, &k, &c, &e};
-  const void* fn = gang_kernel(prec);
-  USAP_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kPThreads), kargs, kPSmemBytes, st));
-  USAP_LAUNCHED();
 }
 
 void launch_nodal_phase(const PhaseArgs& p, int grid, cudaStream_t st) {

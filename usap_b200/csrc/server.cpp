@@ -13,6 +13,7 @@
 // seed.  Completion is read with usap_server_poll / usap_server_wait.
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <condition_variable>
 #include <cstring>
 #include <deque>
@@ -57,19 +58,24 @@ int64_t solve_footprint_bytes(int64_t n, int64_t e, int64_t dense_max, bool weig
   const int64_t graph = (weighted ? 48 : 32) * e + 64 * n + 8 * (e + 1);
   const int64_t state = 72 * n + 160 * n + 112 * e;
   const int64_t tile = 8 * (d + 4) * (d + 4) + 4 * d * ((d + 127) / 128 + 1);
-  const int64_t dt = std::min<int64_t>(d, 4096);
+  // (the float dS has term tables up to a fifth as many edges as cells)
+  const int64_t dt = std::min(d, std::max<int64_t>(4096, static_cast<int64_t>(std::sqrt(5.0 * static_cast<double>(e)))));
   const int64_t tables = float_ds ? 8 * (dt + 4) * (dt + 4) : 0;
   return graph + state + tile + tables + (8ll << 20);
 }
 
 class Server {
- public:
-  Server(const usap_server_config& cfg) : device_(cfg.device) {
+  static int checked_device(int device) {
     int count = 0;
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0)
       throw Error(USAP_ERR_NO_DEVICE, "no CUDA device available");
-    if (device_ < 0 || device_ >= count) throw Error(USAP_ERR_INVALID, "device index out of range");
-    USAP_CUDA(cudaSetDevice(device_));
+    if (device < 0 || device >= count) throw Error(USAP_ERR_INVALID, "device index out of range");
+    USAP_CUDA(cudaSetDevice(device));
+    return device;
+  }
+
+ public:
+  Server(const usap_server_config& cfg) : device_(cfg.device), pool_(checked_device(cfg.device)) {
     size_t free_b = 0, total_b = 0;
     USAP_CUDA(cudaMemGetInfo(&free_b, &total_b));
     budget_ = cfg.memory_budget > 0 ? cfg.memory_budget : static_cast<int64_t>(0.8 * static_cast<double>(free_b));
@@ -78,14 +84,12 @@ class Server {
     const int nw = cfg.workers > 0 ? cfg.workers : std::min(32, 2 * hw);
     // the solver states are created up front, so that a missing or
     // unusable device fails here and not in a worker
-    std::vector<std::unique_ptr<Job>> states;
-    for (int i = 0; i < nw; i++) states.push_back(std::make_unique<Job>(device_));
-    for (int i = 0; i < nw; i++) {
-      workers_.emplace_back([this, st = states[i].release()] {
-        std::unique_ptr<Job> job(st);
-        work(job.get());
-      });
+    for (int i = 0; i < std::min(nw, kSolveSlots); i++) {
+      states_.push_back(std::make_unique<Job>(device_));
+      states_.back()->set_pool(&pool_);
+      free_.push_back(states_.back().get());
     }
+    for (int i = 0; i < nw; i++) workers_.emplace_back([this] { work(); });
   }
 
   ~Server() {
@@ -109,7 +113,6 @@ class Server {
     r->g.dst = r->dst.data();
     r->g.weight = g.weight ? r->w.data() : nullptr;
     r->params = p;
-    r->params.persistent = 0;   // the cooperative kernel would hold every SM
     r->out_assign = out_assign;
     int64_t n = g.n;
     if (n <= 0) {
@@ -176,19 +179,24 @@ class Server {
   }
 
  private:
-  void work(Job* job) {
+  void work() {
     for (;;) {
       std::shared_ptr<Request> r;
+      Job* job = nullptr;
       {
         std::unique_lock<std::mutex> lk(mu_);
-        // arrival order; the oldest waiting request goes first as soon as
-        // its footprint fits in the budget left by the running ones
+        // arrival order; the oldest waiting request goes first as soon as a
+        // solver state is free and its footprint fits in the budget left by
+        // the running ones
         cv_work_.wait(lk, [&] {
-          return (stopping_ && queue_.empty()) || (!queue_.empty() && admitted_ + queue_.front()->bytes <= budget_);
+          return (stopping_ && queue_.empty()) ||
+                 (!queue_.empty() && !free_.empty() && admitted_ + queue_.front()->bytes <= budget_);
         });
         if (queue_.empty()) return;
         r = queue_.front();
         queue_.pop_front();
+        job = free_.back();
+        free_.pop_back();
         admitted_ += r->bytes;
         running_++;
         peak_admitted_ = std::max(peak_admitted_, admitted_);
@@ -222,6 +230,7 @@ class Server {
         std::lock_guard<std::mutex> lk(mu_);
         r->finished = Clock::now();
         r->done = true;
+        free_.push_back(job);
         admitted_ -= r->bytes;
         running_--;
         if (r->status == USAP_OK) completed_++;
@@ -233,11 +242,14 @@ class Server {
   }
 
   int device_;
+  SmPool pool_;   // the SMs that the requests' nodal phases share
   int64_t budget_ = 0;
   std::mutex mu_;
   std::condition_variable cv_work_, cv_done_;
   std::deque<std::shared_ptr<Request>> queue_;
   std::unordered_map<int64_t, std::shared_ptr<Request>> requests_;
+  std::vector<std::unique_ptr<Job>> states_;   // shared by the workers
+  std::vector<Job*> free_;
   std::vector<std::thread> workers_;
   int64_t next_ticket_ = 1;
   int64_t admitted_ = 0, peak_admitted_ = 0;
