@@ -35,13 +35,30 @@ struct TsvStatus {
   int nonunit;
 };
 
-__global__ void k_tsv_count(const char* __restrict__ text, int64_t len, int* __restrict__ counts) {
-  const int64_t base = blockIdx.x * static_cast<int64_t>(kChunk) + threadIdx.x * static_cast<int64_t>(kBytesPerThread);
-  int c = 0;
-  for (int k = 0; k < kBytesPerThread; k++) {
-    const int64_t i = base + k;
-    if (i < len && text[i] == '\n') c++;
+// A thread's 16 bytes of text as bits (bit k: byte base + k is a newline), by
+// one 16-byte load: base is a multiple of 16 and the text starts on an
+// allocation's boundary.  The text's last, incomplete piece is read bytewise.
+__device__ __forceinline__ unsigned newline_bits(const char* __restrict__ text, int64_t len, int64_t base) {
+  unsigned bits = 0;
+  if (base + kBytesPerThread <= len) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(text + base));
+    const unsigned w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const unsigned m = __vcmpeq4(w[k], 0x0a0a0a0au) & 0x01010101u;
+      bits |= ((m * 0x01020408u) >> 24) << (4 * k);   // bits 0, 8, 16, 24 to 0..3 (no two products meet in a bit)
+    }
+  } else {
+    for (int k = 0; k < kBytesPerThread; k++)
+      if (base + k < len && text[base + k] == '\n') bits |= 1u << k;
   }
+  return bits;
+}
+
+__global__ void __launch_bounds__(kThreads) k_tsv_count(const char* __restrict__ text, int64_t len,
+                                                        int* __restrict__ counts) {
+  const int64_t base = blockIdx.x * static_cast<int64_t>(kChunk) + threadIdx.x * static_cast<int64_t>(kBytesPerThread);
+  const int c = __popc(newline_bits(text, len, base));
   typedef cub::BlockReduce<int, kThreads> Reduce;
   __shared__ typename Reduce::TempStorage tmp;
   const int total = Reduce(tmp).Sum(c);
@@ -49,23 +66,17 @@ __global__ void k_tsv_count(const char* __restrict__ text, int64_t len, int* __r
 }
 
 // newline positions in order: block offsets from the scan of the counts
-__global__ void k_tsv_positions(const char* __restrict__ text, int64_t len, const int* __restrict__ offsets,
-                                int64_t* __restrict__ nl) {
+__global__ void __launch_bounds__(kThreads) k_tsv_positions(const char* __restrict__ text, int64_t len,
+                                                            const int* __restrict__ offsets,
+                                                            int64_t* __restrict__ nl) {
   const int64_t base = blockIdx.x * static_cast<int64_t>(kChunk) + threadIdx.x * static_cast<int64_t>(kBytesPerThread);
-  int c = 0;
-  for (int k = 0; k < kBytesPerThread; k++) {
-    const int64_t i = base + k;
-    if (i < len && text[i] == '\n') c++;
-  }
+  unsigned bits = newline_bits(text, len, base);
   typedef cub::BlockScan<int, kThreads> Scan;
   __shared__ typename Scan::TempStorage tmp;
   int before = 0;
-  Scan(tmp).ExclusiveSum(c, before);
-  int64_t o = offsets[blockIdx.x] + before;
-  for (int k = 0; k < kBytesPerThread; k++) {
-    const int64_t i = base + k;
-    if (i < len && text[i] == '\n') nl[o++] = i;
-  }
+  Scan(tmp).ExclusiveSum(__popc(bits), before);
+  for (int64_t o = offsets[blockIdx.x] + static_cast<int64_t>(before); bits; bits &= bits - 1)
+    nl[o++] = base + __ffs(bits) - 1;
 }
 
 __device__ __forceinline__ bool is_space(char c) {
@@ -122,9 +133,14 @@ __device__ __forceinline__ int64_t find_tab(const char* t, int64_t b, int64_t e)
   return b;   // e when there is none
 }
 
-__global__ void k_tsv_parse(const char* __restrict__ text, int64_t len, const int64_t* __restrict__ nl, int64_t lines,
-                            int32_t* __restrict__ src, int32_t* __restrict__ dst, int32_t* __restrict__ w,
-                            TsvStatus* st) {
+// (the largest ids are reduced within a CTA first: an atomic per line would
+// queue them all on one address)
+__global__ void __launch_bounds__(kThreads) k_tsv_parse(const char* __restrict__ text, int64_t len,
+                                                        const int64_t* __restrict__ nl, int64_t lines,
+                                                        int32_t* __restrict__ src, int32_t* __restrict__ dst,
+                                                        int32_t* __restrict__ w, TsvStatus* st) {
+  int max_src = 0, max_id = 0;
+  bool nonunit = false;
   for (int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; k < lines;
        k += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t b = k == 0 ? 0 : nl[k - 1] + 1;
@@ -152,9 +168,24 @@ __global__ void k_tsv_parse(const char* __restrict__ text, int64_t len, const in
     src[k] = static_cast<int32_t>(a - 1);
     dst[k] = static_cast<int32_t>(c - 1);
     w[k] = static_cast<int32_t>(x);
-    atomicMax(&st->max_src, static_cast<int>(a));
-    atomicMax(&st->max_id, static_cast<int>(a > c ? a : c));
-    if (x != 1) st->nonunit = 1;
+    max_src = max(max_src, static_cast<int>(a));
+    max_id = max(max_id, static_cast<int>(a > c ? a : c));
+    nonunit |= x != 1;
+  }
+  __shared__ int s_src, s_id;
+  if (threadIdx.x == 0) s_src = s_id = 0;
+  __syncthreads();
+  max_src = __reduce_max_sync(0xffffffffu, max_src);
+  max_id = __reduce_max_sync(0xffffffffu, max_id);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&s_src, max_src);
+    atomicMax(&s_id, max_id);
+  }
+  if (nonunit) st->nonunit = 1;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    atomicMax(&st->max_src, s_src);
+    atomicMax(&st->max_id, s_id);
   }
 }
 
