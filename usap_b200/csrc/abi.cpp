@@ -166,7 +166,7 @@ usap_status usap_ctx_load_tsv(usap_ctx* ctx, const char* text, int64_t len, int3
     // lists for its own passes (initial blocks, work units)
     usap::HostGraph h;
     usap::TsvEdges t = usap::parse_tsv_device(ctx->job->device(), text ? text : "", len, n, &h);
-    if (t.src.empty()) throw usap::Error(USAP_ERR_INVALID, "graph needs at least one edge");
+    if (t.lines == 0) throw usap::Error(USAP_ERR_INVALID, "graph needs at least one edge");
     ctx->job->load_host(std::move(h));
   });
 }

@@ -323,19 +323,34 @@ std::shared_ptr<GraphResident> load_graph(int device, const usap_graph& in, Host
       USAP_CUDA(cudaMemcpyAsync(*d, v.data(), sizeof(int32_t) * v.size(), cudaMemcpyHostToDevice, st_));
     up_bytes += static_cast<long long>(sizeof(int32_t) * v.size());
   };
-  up(&g.src, h.src);
-  up(&g.dst, h.dst);
-  if (!h.unit) {
-    up(&g.w, h.w);
-    up(&g.out_w, h.out_w);
-    up(&g.in_w, h.in_w);
+  const std::unique_ptr<DeviceLists> dev = std::move(h.dev);
+  if (dev) {   // on the device already (and the work that wrote them waited for)
+    g.src = dev->src;
+    g.dst = dev->dst;
+    g.w = dev->w;
+    g.out_ptr = dev->out_ptr;
+    g.out_idx = dev->out_idx;
+    g.out_w = dev->out_w;
+    g.in_ptr = dev->in_ptr;
+    g.in_idx = dev->in_idx;
+    g.in_w = dev->in_w;
+    g.kout = dev->kout;
+    g.kin = dev->kin;
+  } else {
+    up(&g.src, h.src);
+    up(&g.dst, h.dst);
+    if (!h.unit) {
+      up(&g.w, h.w);
+      up(&g.out_w, h.out_w);
+      up(&g.in_w, h.in_w);
+    }
+    up(&g.out_ptr, h.out_ptr);
+    up(&g.out_idx, h.out_idx);
+    up(&g.in_ptr, h.in_ptr);
+    up(&g.in_idx, h.in_idx);
+    up(&g.kout, h.kout);
+    up(&g.kin, h.kin);
   }
-  up(&g.out_ptr, h.out_ptr);
-  up(&g.out_idx, h.out_idx);
-  up(&g.in_ptr, h.in_ptr);
-  up(&g.in_idx, h.in_idx);
-  up(&g.kout, h.kout);
-  up(&g.kin, h.kin);
   {
     h.chunk_ptr.assign(static_cast<size_t>(n) + 1, 0);
     for (int32_t v = 0; v < n; v++) {
@@ -378,6 +393,7 @@ std::shared_ptr<GraphResident> load_graph(int device, const usap_graph& in, Host
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   gr->g = g;
+  if (dev) dev->owned.clear();   // they are gr's now
   gr->hg = std::move(h);
   gr->hub_ids = std::move(hubs);
   return gr;

@@ -26,6 +26,29 @@ inline int32_t effective_dense_max(const usap_params& p) {
   return p.dense_max > 0 ? p.dense_max : (p.precision == 3 ? 16384 : 4096);
 }
 
+// A graph's arrays that are in device memory already (built there from a parsed
+// TSV): load_graph takes them over instead of uploading the host's copies.
+// Frees what nobody took.
+struct DeviceLists {
+  int32_t *src = nullptr, *dst = nullptr, *w = nullptr;
+  int32_t *out_ptr = nullptr, *out_idx = nullptr, *out_w = nullptr, *kout = nullptr;
+  int32_t *in_ptr = nullptr, *in_idx = nullptr, *in_w = nullptr, *kin = nullptr;
+  std::vector<void*> owned;
+  DeviceLists() = default;
+  DeviceLists(const DeviceLists&) = delete;
+  DeviceLists& operator=(const DeviceLists&) = delete;
+  ~DeviceLists() {
+    if (!owned.empty()) cudaDeviceSynchronize();   // an error path: work on them may be queued
+    for (void* p : owned) cudaFree(p);
+  }
+  // stream-ordered memory, used on other streams only after `st` was waited for
+  int32_t* alloc(int64_t count, cudaStream_t st) {
+    owned.reserve(owned.size() + 1);
+    owned.push_back(dev_alloc(sizeof(int32_t) * count, st));
+    return static_cast<int32_t*>(owned.back());
+  }
+};
+
 struct HostGraph {
   int32_t n = 0;
   int64_t e = 0;
@@ -44,6 +67,7 @@ struct HostGraph {
   // the out/in lists and weighted degrees are filled already (built on the
   // device from a parsed TSV, build_csr_device)
   bool csr_built = false;
+  std::unique_ptr<DeviceLists> dev;   // the same arrays on the device, until load_graph takes them
 };
 
 // _scc + _dfs_itr (graph_parallel.hpp:514-603), host side; scc_prepare
@@ -65,17 +89,17 @@ int32_t compact_labels(const int32_t* init, int32_t n, int32_t* part);
 // are 1; max_src is the reference's N
 struct TsvEdges {
   std::vector<int32_t> src, dst, w;
+  int64_t lines = 0;
   int32_t max_src = 0, max_id = 0;
 };
 // With `graph` given, the parsed edges (0-based, n = the given n or else the
 // largest source id) and their out/in lists, built on the device by
-// build_csr_device, are also returned there.
+// build_csr_device, are returned there instead, on the host and the device.
 TsvEdges parse_tsv_device(int device, const char* text, int64_t len, int32_t n = 0, HostGraph* graph = nullptr);
 // out/in lists and weighted degrees of h's edges (h.n, h.e, h.src, h.unit
-// set) from the same edges in device memory (kernels_csr.cu); alloc
+// set) from the same edges in device memory, h.dev's (kernels_csr.cu); alloc
 // returns stream-ordered device memory freed by the caller
-void build_csr_device(const int32_t* d_src, const int32_t* d_dst, const int32_t* d_w, HostGraph& h,
-                      cudaStream_t st, const std::function<void*(size_t)>& alloc);
+void build_csr_device(HostGraph& h, cudaStream_t st, const std::function<void*(size_t)>& alloc);
 void scan_exclusive_i32(const int32_t* in, int64_t m, int32_t* out, cudaStream_t st,
                         const std::function<void*(size_t)>& alloc);
 // initial blocks on the device (init_mode 2, kernels_init.cu): compact

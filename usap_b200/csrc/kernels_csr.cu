@@ -152,20 +152,17 @@ void scan_exclusive_i32(const int32_t* cnt, int64_t m, int32_t* ptr, cudaStream_
 namespace {
 
 // one side (keyed by `key`): ptr (n + 1), idx and optional weights (e), the
-// weighted degree per key
+// weighted degree per key (n), on the device and the host
 void csr_side(const int32_t* key, const int32_t* val, const int32_t* w, int64_t e, int32_t n, cudaStream_t st,
-              const std::function<void*(size_t)>& alloc, std::vector<int32_t>& h_ptr, std::vector<int32_t>& h_idx,
-              std::vector<int32_t>* h_w, std::vector<int32_t>& h_deg) {
+              const std::function<void*(size_t)>& alloc, int32_t* ptr, int32_t* idx, int32_t* wo, int32_t* deg,
+              std::vector<int32_t>& h_ptr, std::vector<int32_t>& h_idx, std::vector<int32_t>* h_w,
+              std::vector<int32_t>& h_deg) {
   const int64_t m = static_cast<int64_t>(n) + 1;
   int32_t* cnt = static_cast<int32_t*>(alloc(sizeof(int32_t) * m));
-  int32_t* deg = static_cast<int32_t*>(alloc(sizeof(int32_t) * m));
-  int32_t* ptr = static_cast<int32_t*>(alloc(sizeof(int32_t) * m));
   int32_t* cursor = static_cast<int32_t*>(alloc(sizeof(int32_t) * m));
   int32_t* tmp = static_cast<int32_t*>(alloc(sizeof(int32_t) * e));
-  int32_t* idx = static_cast<int32_t*>(alloc(sizeof(int32_t) * e));
-  int32_t* wo = w ? static_cast<int32_t*>(alloc(sizeof(int32_t) * e)) : nullptr;
   USAP_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * m, st));
-  USAP_CUDA(cudaMemsetAsync(deg, 0, sizeof(int32_t) * m, st));
+  USAP_CUDA(cudaMemsetAsync(deg, 0, sizeof(int32_t) * n, st));
   USAP_CUDA(cudaMemsetAsync(cursor, 0, sizeof(int32_t) * m, st));
   k_csr_count<<<grid_for(e, kThreads), kThreads, 0, st>>>(key, w, e, cnt, deg);
   USAP_LAUNCHED();
@@ -188,11 +185,23 @@ void csr_side(const int32_t* key, const int32_t* val, const int32_t* w, int64_t 
 
 }  // namespace
 
-void build_csr_device(const int32_t* d_src, const int32_t* d_dst, const int32_t* d_w, HostGraph& h,
-                      cudaStream_t st, const std::function<void*(size_t)>& alloc) {
-  const int32_t* w = h.unit ? nullptr : d_w;
-  csr_side(d_src, d_dst, w, h.e, h.n, st, alloc, h.out_ptr, h.out_idx, h.unit ? nullptr : &h.out_w, h.kout);
-  csr_side(d_dst, d_src, w, h.e, h.n, st, alloc, h.in_ptr, h.in_idx, h.unit ? nullptr : &h.in_w, h.kin);
+void build_csr_device(HostGraph& h, cudaStream_t st, const std::function<void*(size_t)>& alloc) {
+  DeviceLists& d = *h.dev;
+  const int64_t m = static_cast<int64_t>(h.n) + 1;
+  d.out_ptr = d.alloc(m, st);
+  d.in_ptr = d.alloc(m, st);
+  d.out_idx = d.alloc(h.e, st);
+  d.in_idx = d.alloc(h.e, st);
+  d.kout = d.alloc(h.n, st);
+  d.kin = d.alloc(h.n, st);
+  if (!h.unit) {
+    d.out_w = d.alloc(h.e, st);
+    d.in_w = d.alloc(h.e, st);
+  }
+  csr_side(d.src, d.dst, d.w, h.e, h.n, st, alloc, d.out_ptr, d.out_idx, d.out_w, d.kout, h.out_ptr, h.out_idx,
+           h.unit ? nullptr : &h.out_w, h.kout);
+  csr_side(d.dst, d.src, d.w, h.e, h.n, st, alloc, d.in_ptr, d.in_idx, d.in_w, d.kin, h.in_ptr, h.in_idx,
+           h.unit ? nullptr : &h.in_w, h.kin);
   USAP_CUDA(cudaStreamSynchronize(st));
   bool by_source = true;
   for (int64_t i = 1; i < h.e && by_source; i++) by_source = h.src[i - 1] <= h.src[i];

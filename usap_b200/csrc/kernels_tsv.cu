@@ -214,6 +214,7 @@ TsvEdges parse_tsv_device(int device, const char* text, int64_t len, int32_t n, 
     return p;
   };
   TsvEdges out;
+  auto dev = std::make_unique<DeviceLists>();
   if (len == 0) return out;
   char* d_text = static_cast<char*>(alloc(static_cast<size_t>(len)));
   USAP_CUDA(cudaMemcpyAsync(d_text, text, static_cast<size_t>(len), cudaMemcpyHostToDevice, st));
@@ -242,13 +243,15 @@ TsvEdges parse_tsv_device(int device, const char* text, int64_t len, int32_t n, 
     const int64_t end = len;
     USAP_CUDA(cudaMemcpyAsync(nl + lines - 1, &end, sizeof(int64_t), cudaMemcpyHostToDevice, st));
   }
-  int32_t* dv = static_cast<int32_t*>(alloc(sizeof(int32_t) * 3 * lines));
+  int32_t* d_src = dev->src = dev->alloc(lines, st);
+  int32_t* d_dst = dev->dst = dev->alloc(lines, st);
+  int32_t* d_w = static_cast<int32_t*>(alloc(sizeof(int32_t) * lines));
   TsvStatus* ds = static_cast<TsvStatus*>(alloc(sizeof(TsvStatus)));
   const TsvStatus init{~0ull, 0, 0, 0};
   USAP_CUDA(cudaMemcpyAsync(ds, &init, sizeof(init), cudaMemcpyHostToDevice, st));
   int64_t pb = (lines + kThreads - 1) / kThreads;
   if (pb > 148 * 16) pb = 148 * 16;
-  k_tsv_parse<<<static_cast<int>(pb), kThreads, 0, st>>>(d_text, len, nl, lines, dv, dv + lines, dv + 2 * lines, ds);
+  k_tsv_parse<<<static_cast<int>(pb), kThreads, 0, st>>>(d_text, len, nl, lines, d_src, d_dst, d_w, ds);
   USAP_LAUNCHED();
   TsvStatus hs{};
   USAP_CUDA(cudaMemcpyAsync(&hs, ds, sizeof(hs), cudaMemcpyDeviceToHost, st));
@@ -262,13 +265,14 @@ TsvEdges parse_tsv_device(int device, const char* text, int64_t len, int32_t n, 
   }
   out.src.resize(lines);
   out.dst.resize(lines);
-  USAP_CUDA(cudaMemcpyAsync(out.src.data(), dv, sizeof(int32_t) * lines, cudaMemcpyDeviceToHost, st));
-  USAP_CUDA(cudaMemcpyAsync(out.dst.data(), dv + lines, sizeof(int32_t) * lines, cudaMemcpyDeviceToHost, st));
+  USAP_CUDA(cudaMemcpyAsync(out.src.data(), d_src, sizeof(int32_t) * lines, cudaMemcpyDeviceToHost, st));
+  USAP_CUDA(cudaMemcpyAsync(out.dst.data(), d_dst, sizeof(int32_t) * lines, cudaMemcpyDeviceToHost, st));
   if (hs.nonunit) {
     out.w.resize(lines);
-    USAP_CUDA(cudaMemcpyAsync(out.w.data(), dv + 2 * lines, sizeof(int32_t) * lines, cudaMemcpyDeviceToHost, st));
+    USAP_CUDA(cudaMemcpyAsync(out.w.data(), d_w, sizeof(int32_t) * lines, cudaMemcpyDeviceToHost, st));
   }
   USAP_CUDA(cudaStreamSynchronize(st));
+  out.lines = lines;
   out.max_src = hs.max_src;
   out.max_id = hs.max_id;
   if (graph) {
@@ -285,10 +289,15 @@ TsvEdges parse_tsv_device(int device, const char* text, int64_t len, int32_t n, 
     for (int32_t x : out.w) h.wtot += x;
     if (h.unit) h.wtot = lines;
     if (h.wtot >= (1ll << 24)) throw Error(USAP_ERR_LIMIT, "total edge weight must be below 2^24");
-    h.src = out.src;
-    h.dst = out.dst;
-    h.w = out.w;
-    build_csr_device(dv, dv + lines, dv + 2 * lines, h, st, alloc);
+    h.src = std::move(out.src);
+    h.dst = std::move(out.dst);
+    h.w = std::move(out.w);
+    if (!h.unit) {
+      dev->w = dev->alloc(lines, st);
+      USAP_CUDA(cudaMemcpyAsync(dev->w, d_w, sizeof(int32_t) * lines, cudaMemcpyDeviceToDevice, st));
+    }
+    h.dev = std::move(dev);
+    build_csr_device(h, st, alloc);
   }
   return out;
 }
