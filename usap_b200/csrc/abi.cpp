@@ -286,9 +286,7 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
     auto t0 = std::chrono::steady_clock::now();
     int hw = static_cast<int>(std::thread::hardware_concurrency());
     if (hw <= 0) hw = 8;
-    // the solves' nodal phases share the SMs
     USAP_CUDA(cudaSetDevice(device));
-    usap::SmPool pool(device);
     int W = workers > 0 ? workers : kBatchWorkers;
     W = std::max(1, std::min(W, std::max(njobs, ngraphs)));
     // load every graph once, in parallel
@@ -332,7 +330,9 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
       usap::pool_reserve(device, want);
     }
     std::atomic<int32_t> next{0};
-    std::atomic<long long> launches{0};
+    std::atomic<long long> launches{0}, phases{0};
+    double phase_ms = 0.0;
+    std::mutex phase_mu;
     std::vector<std::thread> th;
     for (int w = 0; w < std::min(std::min(W, usap::kSolveSlots), std::max<int32_t>(njobs, 1)); w++)
       th.emplace_back([&] {
@@ -350,7 +350,7 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
             continue;
           }
           try {
-            job->set_pool(&pool);
+            job->set_concurrent(true);
             job->attach(res[bj.graph]);
             usap_params prm = base;
             prm.seed = bj.seed;
@@ -362,6 +362,11 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
             bj.status = USAP_ERR_INTERNAL;
           }
         }
+        if (job) {
+          phases += job->phases();
+          std::lock_guard<std::mutex> lk(phase_mu);
+          phase_ms += job->phase_ms();
+        }
         job.reset();
         launches += usap::launch_count().kernels - lc0.kernels;
       });
@@ -372,9 +377,9 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
       stats->ms_load = std::chrono::duration<double, std::milli>(t1 - t0).count();
       stats->workers = W;
       stats->kernel_launches = launches.load();
-      stats->gang_launches = pool.launches();
-      stats->gang_phases = pool.launches();
-      stats->ms_gang = pool.ms();
+      stats->gang_launches = phases.load();
+      stats->gang_phases = phases.load();
+      stats->ms_gang = phase_ms;
     }
     for (int32_t j = 0; j < njobs; j++)
       if (jobs[j].status != USAP_OK) throw usap::Error(jobs[j].status, "a batch job failed");

@@ -139,6 +139,7 @@ Job::Job(int device) : device_(device) {
   USAP_CUDA(cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming));
   USAP_CUDA(cudaEventCreateWithFlags(&ev_wait_, cudaEventDisableTiming | cudaEventBlockingSync));
   nodal_configure(device);
+  pool_ = SmPool::of_device(device, nodal_phase_grid(device), nodal_phase_warps());
   USAP_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_ctl_), sizeof(NodalCtl)));
   USAP_CUDA(cudaMallocHost(reinterpret_cast<void**>(&h_ring_), 2 * sizeof(NodalCtl)));
   for (auto& e : ev_sweep_) USAP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -839,7 +840,7 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
   launch_nodal_phase(pa, grid, st_);
   if (timed) USAP_CUDA(cudaEventRecord(e1, st_));
   launch_copy_out(h_ctl_, ctl_, sizeof(NodalCtl), st_);
-  wait(pool_ != nullptr);   // milliseconds, beside other solves' phases
+  wait(concurrent_);   // milliseconds, beside other solves' phases
   if (h_ctl_->bar_err) throw Error(USAP_ERR_INTERNAL, "persistent nodal kernel: a grid barrier timed out");
   float ms = 0;
   if (timed) USAP_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -923,28 +924,19 @@ void Job::emit_trace(int kind, int stage, int itr, int beg, int32_t B, const int
 namespace {
 
 struct PoolSeat {   // the solve is in progress
-  SmPool* p;
+  SmPool& p;
   int64_t batch;
-  PoolSeat(SmPool* pool, int64_t b) : p(pool), batch(b) {
-    if (p) p->enter(batch);
-  }
-  ~PoolSeat() {
-    if (p) p->leave(batch);
-  }
+  PoolSeat(SmPool& pool, int64_t b) : p(pool), batch(b) { p.enter(batch); }
+  ~PoolSeat() { p.leave(batch); }
   PoolSeat(const PoolSeat&) = delete;
   PoolSeat& operator=(const PoolSeat&) = delete;
 };
 
-struct PoolCtas {   // CTAs of one nodal phase: from the pool, or all
-  SmPool* p;
+struct PoolCtas {   // CTAs of one nodal phase
+  SmPool& p;
   int n;
-  std::chrono::steady_clock::time_point t0;
-  PoolCtas(SmPool* pool, int64_t batch, int most) : p(pool), n(pool ? pool->acquire(batch, most) : most) {
-    t0 = std::chrono::steady_clock::now();
-  }
-  ~PoolCtas() {
-    if (p) p->release(n, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
-  }
+  PoolCtas(SmPool& pool, int64_t batch, int most, bool whole) : p(pool), n(pool.acquire(batch, most, whole)) {}
+  ~PoolCtas() { p.release(n); }
   PoolCtas(const PoolCtas&) = delete;
   PoolCtas& operator=(const PoolCtas&) = delete;
 };
@@ -970,7 +962,7 @@ void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res,
   const int32_t maxitr = p.max_num_nodal_itr;
   bs_ = n / p.num_batch_nodal_update;
   if (bs_ < 1) bs_ = 1;
-  const PoolSeat seat(pool_, bs_);
+  const PoolSeat seat(*pool_, bs_);
   const int stats = p.stats ? 1 : 0;
   const bool use_graphs = p.sweep_graphs != 0 && !stats;
   trace_mask_ = p.trace_kinds ? p.trace_kinds : 7;
@@ -1045,11 +1037,14 @@ void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res,
     const double model_d = model_S(n, hg_->e, B);
     trace_prev_moves_ = 0;
     const bool phase_ok = dense && !use_graphs && maxitr > 0 && B <= nodal_phase_max_blocks() && !trace_on(2);
-    const int pgrid = phase_ok && (p.persistent || pool_) ? nodal_phase_grid(device_) : 0;
+    const int pgrid = phase_ok && (p.persistent || concurrent_) ? nodal_phase_grid(device_) : 0;
     const int pmost = p.persistent_ctas > 0 ? std::min(pgrid, static_cast<int>(p.persistent_ctas)) : pgrid;
     if (pgrid > 0) {
-      const PoolCtas ctas(pool_, bs_, pmost);
+      const PoolCtas ctas(*pool_, bs_, pmost, !concurrent_);
+      const auto tp0 = std::chrono::steady_clock::now();
       const float ms = nodal_phase(part, B, stage, seed, W, thr, model_d, maxitr, stats, ctas.n, stats != 0);
+      phases_++;
+      phase_ms_ += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tp0).count();
       d2h += sizeof(NodalCtl);
       if (stats) {
         res->ms_nodal_kernel += ms;

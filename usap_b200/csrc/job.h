@@ -13,6 +13,7 @@
 
 #include "../../include/usap.h"
 #include "engine.h"
+#include "smpool.h"
 
 namespace usap {
 
@@ -181,30 +182,6 @@ std::shared_ptr<GraphResident> load_graph(int device, const usap_graph& in, Host
 // phases fill the SMs.
 constexpr int kSolveSlots = 8;
 
-// The SMs that concurrent solves' nodal phases share (smpool.cpp).
-class SmPool {
- public:
-  explicit SmPool(int device);
-  // a solve with batches of `batch` vertices starts / ends
-  void enter(int64_t batch);
-  void leave(int64_t batch);
-  // CTAs for its next nodal phase, at most `most` (waits for them), given back
-  // with the phase's duration
-  int acquire(int64_t batch, int most);
-  void release(int ctas, double ms);
-  long long launches() const { return launches_; }
-  double ms() const { return ms_; }
-
- private:
-  std::mutex mu_;
-  std::condition_variable cv_;
-  int total_, free_;
-  int64_t live_ = 0;                     // batch vertices of the solves in progress
-  uint64_t next_ = 0, serving_ = 0;      // phases are admitted in arrival order
-  long long launches_ = 0;
-  double ms_ = 0.0;
-};
-
 class Job {
  public:
   explicit Job(int device);
@@ -223,9 +200,13 @@ class Job {
     return hg_ ? *hg_ : empty;
   }
   const std::shared_ptr<GraphResident>& graph() const { return gr_; }
-  // host threads sleep (instead of spinning) while waiting for the device
-  // nodal phases run on SMs of this pool, beside other solves' phases
-  void set_pool(SmPool* p) { pool_ = p; }
+  // one of the solves of a batch or a server: its phases take their share of
+  // the SMs even while it is alone, and its host thread sleeps (instead of
+  // spinning) through them
+  void set_concurrent(bool on) { concurrent_ = on; }
+  // nodal phases run as cooperative launches so far, and their wall time
+  long long phases() const { return phases_; }
+  double phase_ms() const { return phase_ms_; }
   void set_trace(usap_trace_fn fn, void* user) {
     trace_ = fn;
     trace_user_ = user;
@@ -308,7 +289,10 @@ class Job {
   cudaEvent_t ev_wait_ = nullptr;
   cudaEvent_t ev_sweep_[2] = {nullptr, nullptr};   // sweep done + control copied
   NodalCtl* h_ring_ = nullptr;                     // pinned, two control copies
-  SmPool* pool_ = nullptr;
+  std::shared_ptr<SmPool> pool_;                   // the device's
+  bool concurrent_ = false;
+  long long phases_ = 0;
+  double phase_ms_ = 0.0;
   void wait(bool block = false);
   std::shared_ptr<GraphResident> gr_;
   const HostGraph* hg_ = nullptr;

@@ -65,17 +65,13 @@ int64_t solve_footprint_bytes(int64_t n, int64_t e, int64_t dense_max, bool weig
 }
 
 class Server {
-  static int checked_device(int device) {
+ public:
+  Server(const usap_server_config& cfg) : device_(cfg.device) {
     int count = 0;
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0)
       throw Error(USAP_ERR_NO_DEVICE, "no CUDA device available");
-    if (device < 0 || device >= count) throw Error(USAP_ERR_INVALID, "device index out of range");
-    USAP_CUDA(cudaSetDevice(device));
-    return device;
-  }
-
- public:
-  Server(const usap_server_config& cfg) : device_(cfg.device), pool_(checked_device(cfg.device)) {
+    if (device_ < 0 || device_ >= count) throw Error(USAP_ERR_INVALID, "device index out of range");
+    USAP_CUDA(cudaSetDevice(device_));
     size_t free_b = 0, total_b = 0;
     USAP_CUDA(cudaMemGetInfo(&free_b, &total_b));
     budget_ = cfg.memory_budget > 0 ? cfg.memory_budget : static_cast<int64_t>(0.8 * static_cast<double>(free_b));
@@ -86,7 +82,7 @@ class Server {
     // unusable device fails here and not in a worker
     for (int i = 0; i < std::min(nw, kSolveSlots); i++) {
       states_.push_back(std::make_unique<Job>(device_));
-      states_.back()->set_pool(&pool_);
+      states_.back()->set_concurrent(true);
       free_.push_back(states_.back().get());
     }
     for (int i = 0; i < nw; i++) workers_.emplace_back([this] { work(); });
@@ -242,7 +238,6 @@ class Server {
   }
 
   int device_;
-  SmPool pool_;   // the SMs that the requests' nodal phases share
   int64_t budget_ = 0;
   std::mutex mu_;
   std::condition_variable cv_work_, cv_done_;
