@@ -69,14 +69,15 @@ std::mutex g_dlog_mu[kMaxDevices];
 std::shared_ptr<const DeviceLogTable> g_dlog[kMaxDevices];
 }  // namespace
 
-std::shared_ptr<const DeviceLogTable> device_log_table(int device, int64_t max_k, int64_t* uploaded) {
+std::shared_ptr<const DeviceLogTable> device_log_table(int device, int64_t max_k, int64_t* uploaded,
+                                                       int64_t grow_to) {
   if (uploaded) *uploaded = 0;
   if (device < 0 || device >= kMaxDevices) throw Error(USAP_ERR_INVALID, "device index out of range");
   std::lock_guard<std::mutex> lk(g_dlog_mu[device]);
   std::shared_ptr<const DeviceLogTable>& cur = g_dlog[device];
   if (cur && cur->size > max_k) return cur;
   // grow geometrically so that a stream of slightly larger graphs uploads rarely
-  const int64_t size = std::max<int64_t>(max_k + 1, cur ? 2 * cur->size : max_k + 1);
+  const int64_t size = std::max<int64_t>(max_k + 1, cur ? std::min(2 * cur->size, grow_to) : 0);
   const std::shared_ptr<const std::vector<double>> host = log_table(size - 1);
   auto t = std::make_shared<DeviceLogTable>();
   USAP_CUDA(cudaSetDevice(device));

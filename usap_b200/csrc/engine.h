@@ -93,8 +93,10 @@ struct DeviceLogTable {
   ~DeviceLogTable();
 };
 // the device's table with at least max_k + 1 entries; *uploaded = bytes
-// copied to the device by this call (0 when the current table was enough)
-std::shared_ptr<const DeviceLogTable> device_log_table(int device, int64_t max_k, int64_t* uploaded);
+// copied to the device by this call (0 when the current table was enough); a
+// table that grows takes up to grow_to entries for later calls
+std::shared_ptr<const DeviceLogTable> device_log_table(int device, int64_t max_k, int64_t* uploaded,
+                                                       int64_t grow_to = int64_t(1) << 24);
 
 // Dense block matrix view: M[x*ld + y], transposed copy Mt[y*ld + x], and
 // per-row chunk sums CS[u*cld + c] of M[u,i]+M[i,u] over blocks

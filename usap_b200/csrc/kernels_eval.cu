@@ -221,9 +221,12 @@ int count_grid(int64_t n) {
   return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((n + kCountItems - 1) / kCountItems, 148 * 2)));
 }
 
-// entries up to which scores use the device's shared log table: as many as the
-// heaviest graph (total weight below 2^24) keeps there
-constexpr int64_t kSharedLogs = int64_t(1) << 24;
+// Vertices below which a call's scores are enqueued at once and read the
+// device's shared log table, which they grow up to that many entries (64 MiB on
+// the device).  Above, a call learns first how many vertices count, and brings
+// a larger table than that in memory of its own: the device passes take
+// milliseconds there, and the shared table lives as long as the process.
+constexpr int64_t kSharedLogs = int64_t(1) << 22;
 
 }  // namespace
 
@@ -262,28 +265,41 @@ void evaluate_device(const int32_t* truth, const int32_t* given, int64_t n, int 
   USAP_CUDA(cudaMemsetAsync(base, 0, sizeof(Back) + sizeof(unsigned) * 2 * kSmallCells, st));
   k_eval_labels<<<count_grid(n), kCountThreads, 0, st>>>(n, truth, given, &head->info);
   USAP_LAUNCHED();
-  USAP_CUDA(cudaFuncSetAttribute(k_eval_count_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kSmallSmem)));
-  k_eval_count_small<<<count_grid(n), kCountThreads, kSmallSmem, st>>>(n, truth, given, &head->info, table, rows, cols);
-  USAP_LAUNCHED();
   std::shared_ptr<const DeviceLogTable> logs;
   std::shared_ptr<const std::vector<double>> Lp;
+  auto logs_to = [&](int64_t k) -> const double* {
+    if (k < kSharedLogs) {
+      logs = device_log_table(device, k, nullptr, kSharedLogs);
+      return logs->L;
+    }
+    Lp = log_table(k);
+    double* up = static_cast<double*>(alloc(sizeof(double) * (k + 1)));
+    USAP_CUDA(cudaMemcpyAsync(up, Lp->data(), sizeof(double) * (k + 1), cudaMemcpyHostToDevice, st));
+    return up;
+  };
   const double* L = nullptr;
-  if (n < kSharedLogs) {
-    logs = device_log_table(device, n, nullptr);
-    L = logs->L;
-  } else {
-    Lp = log_table(n);
-    double* up = static_cast<double*>(alloc(sizeof(double) * (n + 1)));
-    USAP_CUDA(cudaMemcpyAsync(up, Lp->data(), sizeof(double) * (n + 1), cudaMemcpyHostToDevice, st));
-    L = up;
-  }
-  k_eval_sums<<<grid_for(2 * kSmallCells + 1), kThreads, 0, st>>>(&head->info, true, table, rows, cols, L, &head->sums);
-  USAP_LAUNCHED();
   Back back;
-  USAP_CUDA(cudaMemcpyAsync(&back, base, sizeof(back), cudaMemcpyDeviceToHost, st));
-  USAP_CUDA(cudaStreamSynchronize(st));
-  const LabelInfo& li = back.head.info;
+  auto small_scores = [&](int64_t k) {   // log k of every count needed
+    USAP_CUDA(cudaFuncSetAttribute(k_eval_count_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(kSmallSmem)));
+    k_eval_count_small<<<count_grid(n), kCountThreads, kSmallSmem, st>>>(n, truth, given, &head->info, table, rows,
+                                                                         cols);
+    USAP_LAUNCHED();
+    L = logs_to(k);
+    k_eval_sums<<<grid_for(2 * kSmallCells + 1), kThreads, 0, st>>>(&head->info, true, table, rows, cols, L,
+                                                                    &head->sums);
+    USAP_LAUNCHED();
+    USAP_CUDA(cudaMemcpyAsync(&back, base, sizeof(back), cudaMemcpyDeviceToHost, st));
+    USAP_CUDA(cudaStreamSynchronize(st));
+  };
+  const bool at_once = n < kSharedLogs;
+  if (at_once) {
+    small_scores(n);
+  } else {
+    USAP_CUDA(cudaMemcpyAsync(&back.head, head, sizeof(EvalHead), cudaMemcpyDeviceToHost, st));
+    USAP_CUDA(cudaStreamSynchronize(st));
+  }
+  const LabelInfo li = back.head.info;
   if (li.bad & 1) throw Error(USAP_ERR_INVALID, "given labels must be >= 0 and truth labels >= -1");
   const int b1 = li.b1, b2 = li.b2;
   const int64_t N = static_cast<int64_t>(li.known);
@@ -292,6 +308,10 @@ void evaluate_device(const int32_t* truth, const int32_t* given, int64_t n, int 
   const int64_t cells = static_cast<int64_t>(b1) * b2;
   if (cells > kMaxCells) throw Error(USAP_ERR_LIMIT, "contingency table above 2^26 cells");
   const int m = b1 > b2 ? b1 : b2;
+  if (!at_once) {
+    if (eval_small(li)) small_scores(N);
+    else L = logs_to(N);
+  }
   EvalSums e = back.head.sums;
   std::vector<unsigned> big;
   const unsigned* t = back.table;
