@@ -228,8 +228,8 @@ struct NodalArgs {
   float* Trow;            // M[b,i] log(M[b,i] / (d_in[i] d_out[b]))
   float* Tcol;            // M[i,b] log(M[i,b] / (d_out[i] d_in[b]))
   int tld;
-  int sparse;             // precision mode 3: skip the tile's empty cells (float_ds_sparse)
   int coop;               // precision mode 3, persistent kernels: a CTA evaluates its float dS together
+  int sparse;             // ... skipping the tile's empty cells (float_ds_sparse)
   int hub_units;          // ... and a warp proposes for any vertex (no hub CTAs)
 };
 
@@ -302,9 +302,9 @@ void launch_merge_relabel(int n, int B, int32_t* part, const int32_t* root, int3
 void nodal_configure(int device);
 // grid of the persistent nodal kernel on `device` (0: not available)
 int nodal_phase_grid(int device);
-// precision mode 3: whether the float dS packs the non-zero cells of its rows
-// before it evaluates terms (a tile of B x B cells, `e` edges)
-bool float_ds_sparse(int64_t e, int32_t B, bool coop);
+// precision mode 3, persistent kernel: whether the float dS packs the non-zero
+// cells of its rows before it evaluates terms (a tile of B x B cells, `e` edges)
+bool float_ds_sparse(int64_t e, int32_t B);
 int nodal_phase_warps();   // warps of one of its CTAs
 // largest B whose hub tables fit the persistent kernel's shared memory
 int nodal_phase_max_blocks();

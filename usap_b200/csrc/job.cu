@@ -668,8 +668,8 @@ NodalArgs Job::nodal_args(int32_t* part, int32_t B, int32_t beg, int32_t end, ui
   a.Trow = nullptr;
   a.Tcol = nullptr;
   a.tld = 0;
-  a.sparse = prec_ == 3 && float_ds_sparse(g_.e, B, false) ? 1 : 0;
   a.coop = 0;
+  a.sparse = 0;
   a.hub_units = 0;
   if (stats == 2) {   // replay: per-vertex proposals
     a.prop_s = rp_s_;
@@ -806,7 +806,7 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
   bar_test_timeout_ns_ = 0;
   if (prec_ == 3) {
     pa.a.coop = 1;
-    pa.a.sparse = float_ds_sparse(g_.e, B, true) ? 1 : 0;
+    pa.a.sparse = float_ds_sparse(g_.e, B) ? 1 : 0;
     // a warp's table counts 16 bits a block and direction; beyond 2048
     // neighbours a CTA is faster than a warp
     pa.a.hub_units = !pa.a.shadow && B <= 768 && g_.maxk < 65536 && g_.maxdeg <= 2048;

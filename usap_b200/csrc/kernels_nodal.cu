@@ -691,147 +691,11 @@ __device__ __noinline__ float ref32_nodal(const Ops ops, const int32_t* __restri
   return dS;
 }
 
-// --- the same float dS on a sparse tile -----------------------------------------
-// One proposal by a whole warp.  The rows are read 64 blocks at a time (two
-// per lane), the non-zero entries of the four rows are packed into the
-// warp's queue in the chain's order, and whenever 32 are queued each lane
-// evaluates one term: empty cells cost a compare instead of a term and four
-// additions.
-constexpr int kQueueInts = 2 * (32 + 256) + 32;   // the queue, then a run's terms
-constexpr int kQueue = 32 + 256;   // entries: fewer than 32 left over, and up to 256 of 64 blocks
-
-// a run of 32 (or, at the end, n < 32) terms added to or subtracted from the chain
-__device__ __forceinline__ float ref32_run(float dS, float t, bool sub, float* buf, int lane) {
-  buf[lane] = t;
-  __syncwarp();
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const float4 x = reinterpret_cast<const float4*>(buf)[j];
-    if (sub) dS = __fsub_rn(__fsub_rn(__fsub_rn(__fsub_rn(dS, x.x), x.y), x.z), x.w);
-    else dS = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(dS, x.x), x.y), x.z), x.w);
-  }
-  __syncwarp();
-  return dS;
-}
-
-// One pass (old-state terms added, or new-state terms subtracted) over the
-// rows.  An entry
-// holds the count and, for its row's factor, the block's degree (below
-// 2^24) with the row's number above it.
-template <class Ops, bool kNew>
-__device__ __forceinline__ float ref32_sparse_pass(float dS, const Ops& ops, const int32_t* __restrict__ din_p,
-                                                   const int32_t* __restrict__ dout_p, const Pend& q,
-                                                   const int* key, const int* two, const int* twi, int2* queue,
-                                                   float* buf, int lane) {
-  using LDT = typename Ops::LdT;
-  const int B = ops.B, r = q.r, s = q.s;
-  const int cap = q.cap, lg = q.lg;
-  const float4 ff = kNew ? q.fn : q.fo;
-  const int* mr = ops.v.M + static_cast<long long>(r) * ops.v.ld;
-  const int* ms = ops.v.M + static_cast<long long>(s) * ops.v.ld;
-  const int* tr = ops.v.Mt + static_cast<long long>(r) * ops.v.ld;
-  const int* ts = ops.v.Mt + static_cast<long long>(s) * ops.v.ld;
-  int2 nx[6];
-  auto load = [&](int i) {
-    const int2 z = make_int2(0, 0);
-    const bool in = i < B;   // rows are padded to an even number of columns with zeros
-    nx[0] = in ? LDT::ld(reinterpret_cast<const int2*>(mr + i)) : z;
-    nx[1] = in ? LDT::ld(reinterpret_cast<const int2*>(ms + i)) : z;
-    nx[2] = in ? LDT::ld(reinterpret_cast<const int2*>(tr + i)) : z;
-    nx[3] = in ? LDT::ld(reinterpret_cast<const int2*>(ts + i)) : z;
-    // (the degree arrays are only as long as there are blocks)
-    nx[4] = in ? make_int2(LDT::ld(din_p + i), i + 1 < B ? LDT::ld(din_p + i + 1) : 0) : z;
-    nx[5] = in ? make_int2(LDT::ld(dout_p + i), i + 1 < B ? LDT::ld(dout_p + i + 1) : 0) : z;
-  };
-  int queued = 0;
-  auto run = [&](int head, int n) {   // the n <= 32 entries at `head`
-    int2 e = make_int2(0, 0);
-    if (lane < n) e = queue[head + lane];
-    const int j = e.y >> 24;
-    const float fa = (j & 1) ? ff.y : ff.x, fb = (j & 1) ? ff.w : ff.z;
-    dS = ref32_run(dS, ref_term_nz(e.x, ref_factor(e.y & 0xffffff), (j & 2) ? fb : fa), kNew, buf, lane);
-  };
-  load(2 * lane);
-  for (int base = 0; base < B; base += 64) {
-    const int i = base + 2 * lane;
-    int x[8] = {nx[0].x, nx[1].x, nx[2].x, nx[3].x, nx[0].y, nx[1].y, nx[2].y, nx[3].y};
-    const int di[2] = {nx[4].x, nx[4].y}, dn[2] = {nx[5].x, nx[5].y};
-    load(i + 64);
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const bool rs = i + k == r || i + k == s;   // columns (new: rows too) skip blocks r and s
-      if (rs) x[4 * k + 2] = x[4 * k + 3] = 0;
-      if (kNew) {
-        if (rs) x[4 * k] = x[4 * k + 1] = 0;
-        // v's edges towards block i are part of M[r,i] (out) and M[i,r] (in)
-        if (x[4 * k] > 0) {
-          const int w = table_lookup_wo(key, two, cap, lg, i + k);
-          x[4 * k] -= w;
-          x[4 * k + 1] += w;
-        }
-        if (x[4 * k + 2] > 0) {
-          const int w = table_lookup_wo(key, twi, cap, lg, i + k);
-          x[4 * k + 2] -= w;
-          x[4 * k + 3] += w;
-        }
-      }
-    }
-    int cnt = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) cnt += x[k] != 0;
-    if (!__any_sync(0xffffffffu, cnt != 0)) continue;
-    const int incl = warp_incl_scan(cnt, lane);
-    int at = queued + incl - cnt;
-    if (cnt) {
-#pragma unroll
-      for (int k = 0; k < 2; k++) {
-        if (x[4 * k]) queue[at++] = make_int2(x[4 * k], di[k]);
-        if (x[4 * k + 1]) queue[at++] = make_int2(x[4 * k + 1], di[k] | 1 << 24);
-        if (x[4 * k + 2]) queue[at++] = make_int2(x[4 * k + 2], dn[k] | 2 << 24);
-        if (x[4 * k + 3]) queue[at++] = make_int2(x[4 * k + 3], dn[k] | 3 << 24);
-      }
-    }
-    queued += __shfl_sync(0xffffffffu, incl, 31);
-    __syncwarp();
-    int head = 0;
-    for (; queued - head >= 32; head += 32) run(head, 32);
-    if (head) {   // the rest to the front
-      queued -= head;
-      int2 e = make_int2(0, 0);
-      if (lane < queued) e = queue[head + lane];
-      __syncwarp();
-      if (lane < queued) queue[lane] = e;
-      __syncwarp();
-    }
-  }
-  if (queued) run(0, queued);
-  return dS;
-}
-
-template <class Ops>
-__device__ __noinline__ float ref32_sparse(const Ops ops, const int32_t* __restrict__ din_p,
-                                           const int32_t* __restrict__ dout_p, const Pend& q, const int* key,
-                                           const int* two, const int* twi, int2* queue, float* buf) {
-  const int lane = threadIdx.x & 31;
-  float dS = ref32_sparse_pass<Ops, false>(0.0f, ops, din_p, dout_p, q, key, two, twi, queue, buf, lane);
-  dS = ref32_corner(dS, q);
-  return ref32_sparse_pass<Ops, true>(dS, ops, din_p, dout_p, q, key, two, twi, queue, buf, lane);
-}
-
-template <class Ops>
-constexpr bool kHasTile = false;
-template <class L, int P, class T>
-constexpr bool kHasTile<DenseOpsT<L, P, T>> = true;
-
-// The float dS of a proposal by a whole warp, hashed neighbour blocks.  buf:
-// 128 floats (a dense tile); queue: kQueueInts ints (a sparse one).
+// The float dS of a proposal by a whole warp, hashed neighbour blocks (buf:
+// 128 floats).
 template <class Ops>
 __device__ __forceinline__ float ref32_eval(const NodalArgs& a, const Ops& ops, const Pend& q, const int* key,
-                                            const int* two, const int* twi, int2* queue, float* buf) {
-  if constexpr (kHasTile<Ops>) {
-    if (a.sparse)
-      return ref32_sparse<Ops>(ops, a.din, a.dout, q, key, two, twi, queue, reinterpret_cast<float*>(queue + kQueue));
-  }
+                                            const int* two, const int* twi, float* buf) {
   return ref32_nodal<Ops, 32>(ops, a.din, a.dout, a.Trow, a.Tcol, a.tld, q, key, two, twi, buf);
 }
 
@@ -1201,12 +1065,17 @@ __device__ __forceinline__ bool group_vertex(const NodalArgs& a, const Ops& ops,
 }
 
 // One warp per vertex of degree <= kHubDegree; 5 CTAs per SM so that a
-// batch of the bench workload (N/10 = 5000 vertices) runs in one wave.
+// batch of the bench workload (N/10 = 5000 vertices) runs in one wave.  The
+// float dS evaluates whole rows: the packing of coop_eval_sparse saves terms but
+// adds latency to a warp that has a proposal of its own, and its queue takes
+// shared memory from the fifth CTA and the L1 (N = 20000, per-batch launches:
+// 141 ms a solve with it up to two edges a cell, 111 ms without; N = 50000: 251
+// and 221 ms; N = 3000 from one block per vertex: 245 and 235 ms).
 template <class Ops>
 __global__ void __launch_bounds__(kThreads, 5) k_nodal_propose(NodalArgs a, Ops ops) {
   __shared__ int s_tab[kWarps][3 * kHCap];
-  // occupied slots other than r, s; then the float dS's terms, or its queue
-  __shared__ __align__(16) int s_list[kWarps][kQueueInts];
+  // occupied slots other than r, s; then the float dS's terms
+  __shared__ __align__(16) int s_list[kWarps][kHubDegree];
   __shared__ Pend s_pend[Ops::kP == 3 ? kWarps : 1];
   __shared__ CtaTally s_tally;
   if (a.ctl->done) return;   // written by earlier launches only
@@ -1224,7 +1093,7 @@ __global__ void __launch_bounds__(kThreads, 5) k_nodal_propose(NodalArgs a, Ops 
     if constexpr (Ops::kP == 3) {
       if (live) {   // warp-uniform
         const float f = ref32_eval(a, ops, s_pend[wib], tab, tab + kHCap, tab + 2 * kHCap,
-                                   reinterpret_cast<int2*>(s_list[wib]), reinterpret_cast<float*>(s_list[wib]));
+                                   reinterpret_cast<float*>(s_list[wib]));
         if (lane == 0) close_vertex<Ops>(a, s_pend[wib], f, &s_tally, &my_bytes);
         __syncwarp();
       }
@@ -1252,11 +1121,11 @@ struct HubShared {
 // region's end); each thread loads four neighbours at once, and up to four
 // occupied slots at once for the terms.  In precision 3 the proposal is left
 // in pl's first entry, or, without a list, warp 0 evaluates
-// its float dS (chain: kQueueInts ints).
+// its float dS (chain: 128 floats).
 template <class Ops, int NT>
 __device__ __forceinline__ void hub_vertex(const NodalArgs& a, const Ops& ops, int v, uint32_t itr, int* stab,
                                            int scap, HubShared<NT / 32>* sh, unsigned long long* my_bytes,
-                                           int* chain, PendList* pl) {
+                                           float* chain, PendList* pl) {
   using LD = typename Ops::Ld;
   using LDT = typename Ops::LdT;
   constexpr int NW = NT / 32;
@@ -1439,7 +1308,7 @@ __device__ __forceinline__ void hub_vertex(const NodalArgs& a, const Ops& ops, i
       }
       __syncwarp();
       if (!pl)
-        f = ref32_eval(a, ops, q, key, two, twi, reinterpret_cast<int2*>(chain), reinterpret_cast<float*>(chain));
+        f = ref32_eval(a, ops, q, key, two, twi, chain);
     }
     // (a hub's exact value is a CTA-parallel sum over its slots and is
     // always evaluated; without the shadow it is not reported, as for the
@@ -1462,7 +1331,7 @@ __global__ void __launch_bounds__(kHubThreads) k_nodal_propose_hub(NodalArgs a, 
                                                                   int hub_lo, int hub_hi, int smem_cap) {
   extern __shared__ __align__(16) int dyn[];
   __shared__ HubShared<kHubWarps> sh;
-  __shared__ __align__(16) int s_chain[Ops::kP == 3 ? kQueueInts : 1];
+  __shared__ __align__(16) float s_chain[Ops::kP == 3 ? 128 : 1];
   if (a.ctl->done) return;
   const uint32_t itr = static_cast<uint32_t>(a.ctl->itr);
   unsigned long long my_bytes = 0;
@@ -1976,6 +1845,7 @@ constexpr int kDeltaGlobalMinB = 256;     // from this B the phase kernel's appl
 // hub region stages the cooperative float dS
 constexpr int kSnapMaxB = 88;
 constexpr int kSnapSlots = 256;   // >= a hub table's capacity for B <= kSnapMaxB (2 * B rounded up to a power of 2)
+static_assert(kHubDegree >= 128, "the float dS's terms outgrow a warp's list");
 static_assert(kMaxPend == 2 * kPWarps, "a wave's proposals outgrow the list");
 static_assert(3 * kSnapSlots + 2 * kSnapMaxB * kSnapMaxB + 3 * kSnapMaxB + 2 * kMaxPend * (4 * 16 + 4) <= 3 * kPHubSlots,
               "chunks of 16 blocks of a full list fit beside the tile copy");
@@ -2714,15 +2584,10 @@ int nodal_phase_grid(int device) {
 }
 
 // The line: per 64 blocks packing costs what it saves when about a fifth of
-// the cells are filled (coop; batches of N = 20000 at B = 1227, e = 0.2 cells:
-// 91 us packed, 87 us whole; N = 50000 at B = 1526, 0.33: 385 against 294 us;
-// N = 4999 at B = 625, 0.2: 26 against 33 us).  A single warp also saves the
-// additions that every lane repeats: until two edges a cell (N = 50000, B =
-// 763, 1.3: 230 us packed, 259 us whole).
-bool float_ds_sparse(int64_t e, int32_t B, bool coop) {
-  const int64_t cells = static_cast<int64_t>(B) * B;
-  return B > kSnapMaxB && (coop ? 5 * e < cells : e < 2 * cells);
-}
+// the cells are filled (batches of N = 20000 at B = 1227, e = 0.2 cells: 91 us
+// packed, 87 us whole; N = 50000 at B = 1526, 0.33: 385 against 294 us; N = 4999
+// at B = 625, 0.2: 26 against 33 us).
+bool float_ds_sparse(int64_t e, int32_t B) { return B > kSnapMaxB && 5 * e < static_cast<int64_t>(B) * B; }
 
 int nodal_phase_warps() { return kPWarps; }
 
