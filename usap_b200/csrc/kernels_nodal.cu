@@ -1072,7 +1072,7 @@ __device__ __forceinline__ bool group_vertex(const NodalArgs& a, const Ops& ops,
 // 141 ms a solve with it up to two edges a cell, 111 ms without; N = 50000: 251
 // and 221 ms; N = 3000 from one block per vertex: 245 and 235 ms).
 template <class Ops>
-__global__ void __launch_bounds__(kThreads, 5) k_nodal_propose(NodalArgs a, Ops ops) {
+__global__ void __launch_bounds__(kThreads, 4) k_nodal_propose(NodalArgs a, Ops ops) {
   __shared__ int s_tab[kWarps][3 * kHCap];
   // occupied slots other than r, s; then the float dS's terms
   __shared__ __align__(16) int s_list[kWarps][kHubDegree];
