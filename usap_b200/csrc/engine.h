@@ -63,10 +63,16 @@ LaunchCount& launch_count();
     ::usap::launch_count().cub++;                \
   } while (0)
 
-// Vertices whose degree exceeds kHubDegree are proposed by a whole CTA;
-// its neighbour-block hash holds up to kHubSmemSlots entries in shared
-// memory (3 ints per slot), larger ones use the vertex's global region.
+// Vertices whose degree exceeds kHubDegree (in the persistent kernel) or
+// kBatchHubDegree (per-batch launches) are proposed by a whole CTA; its
+// neighbour-block hash holds up to kHubSmemSlots entries in shared memory (3
+// ints per slot), larger ones use the vertex's global region.  In the
+// persistent kernel a hub holds up a wave; a per-batch launch's hubs run beside
+// its other vertices, and a warp with fewer neighbours a lane is faster (exact
+// FP64 on the sorted views, N = 20000: 138 ms a solve at 128, 147 ms at 192; N =
+// 50000: 177 and 180 ms).
 constexpr int kHubDegree = 192;
+constexpr int kBatchHubDegree = 128;
 constexpr int kPairDegree = 64;   // two vertices up to this degree share a warp (a half-warp each)
 constexpr int kHubSmemSlots = 16384;
 // the persistent kernels' hub table (shared memory): hubs whose table is

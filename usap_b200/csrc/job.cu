@@ -278,13 +278,14 @@ std::shared_ptr<GraphResident> load_graph(int device, const usap_graph& in, Host
   scc_prepare(h);
   // per-vertex global hash regions for degrees beyond the shared-memory table
   std::vector<int64_t> hi_off(n, -1);
-  std::vector<int32_t> hubs;
+  std::vector<int32_t> hubs, batch_hubs;
   int64_t hi_slots = 0;
   int32_t maxdeg = 0, maxk = 0;
   for (int32_t v = 0; v < n; v++) {
     int deg = (h.out_ptr[v + 1] - h.out_ptr[v]) + (h.in_ptr[v + 1] - h.in_ptr[v]);
     maxdeg = std::max(maxdeg, deg);
     maxk = std::max(maxk, std::max(h.kout[v], h.kin[v]));
+    if (deg > kBatchHubDegree) batch_hubs.push_back(v);
     if (deg > kHubDegree) {
       hubs.push_back(v);
       int cap = 1 << hash_lg(deg);
@@ -380,11 +381,14 @@ std::shared_ptr<GraphResident> load_graph(int device, const usap_graph& in, Host
   dalloc(&g.hi_off, n);
   USAP_CUDA(cudaMemcpyAsync(g.hi_off, hi_off.data(), sizeof(int64_t) * n, cudaMemcpyHostToDevice, st_));
   up_bytes += static_cast<long long>(log_bytes + sizeof(int64_t) * n +
-                                     sizeof(int32_t) * hubs.size());
+                                     sizeof(int32_t) * (hubs.size() + batch_hubs.size()));
   g.hi_slots = hi_slots;
-  dalloc(&gr->hubs_dev, hubs.size());
-  if (!hubs.empty())
-    USAP_CUDA(cudaMemcpyAsync(gr->hubs_dev, hubs.data(), sizeof(int32_t) * hubs.size(), cudaMemcpyHostToDevice, st_));
+  std::vector<int32_t> both(hubs);
+  both.insert(both.end(), batch_hubs.begin(), batch_hubs.end());
+  dalloc(&gr->hubs_dev, both.size());
+  gr->batch_hubs_dev = gr->hubs_dev + hubs.size();
+  if (!both.empty())
+    USAP_CUDA(cudaMemcpyAsync(gr->hubs_dev, both.data(), sizeof(int32_t) * both.size(), cudaMemcpyHostToDevice, st_));
   USAP_CUDA(cudaEventRecord(e1, st_));
   USAP_CUDA(cudaStreamSynchronize(st_));
   float ms = 0;
@@ -397,6 +401,7 @@ std::shared_ptr<GraphResident> load_graph(int device, const usap_graph& in, Host
   if (dev) dev->owned.clear();   // they are gr's now
   gr->hg = std::move(h);
   gr->hub_ids = std::move(hubs);
+  gr->batch_hub_ids = std::move(batch_hubs);
   return gr;
 }
 
@@ -472,8 +477,8 @@ void Job::attach(std::shared_ptr<GraphResident> gr) {
 
 HubList Job::hubs_for(int32_t beg, int32_t end, int32_t B) const {
   HubList hl;
-  const std::vector<int32_t>& hub_ids = gr_->hub_ids;
-  hl.ids = gr_->hubs_dev;
+  const std::vector<int32_t>& hub_ids = gr_->batch_hub_ids;
+  hl.ids = gr_->batch_hubs_dev;
   hl.lo = static_cast<int>(std::lower_bound(hub_ids.begin(), hub_ids.end(), beg) - hub_ids.begin());
   hl.hi = static_cast<int>(std::lower_bound(hub_ids.begin(), hub_ids.end(), end) - hub_ids.begin());
   int cap = 32;

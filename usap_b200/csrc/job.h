@@ -166,6 +166,8 @@ struct GraphResident {
   GraphDev g;                      // hkey/hwo/hwi belong to the jobs
   std::vector<int32_t> hub_ids;    // vertices of degree > kHubDegree, ascending
   int32_t* hubs_dev = nullptr;
+  std::vector<int32_t> batch_hub_ids;   // the same beyond kBatchHubDegree
+  const int32_t* batch_hubs_dev = nullptr;   // (behind hubs_dev's)
   double h2d_ms = 0;
   long long h2d_bytes = 0;
 };

@@ -6,9 +6,9 @@
 // scratch rows are cleared and scanned); the update task (:433-458) applies
 // the buffered moves, rebuilds M from scratch and tests convergence.
 //
-// Here one warp proposes for one vertex (one CTA for vertices of degree
-// above kHubDegree, so a hub does not set the batch's tail; up to that, and
-// in precision 3 mostly beyond, a warp is faster).  The target is
+// Here one warp proposes for one vertex (one CTA for vertices of a degree
+// above kHubDegree or kBatchHubDegree, so a hub does not set the batch's tail;
+// up to that, and in precision 3 mostly beyond, a warp is faster).  The target is
 // drawn in block-id order: on the dense tile through per-row chunk sums of
 // M[u,:]+M[:,u] (chunks of 128 blocks, kept current by the same delta
 // updates as M), on the sparse views by binary search of cumulative counts.
@@ -831,16 +831,12 @@ __device__ __forceinline__ void close_vertex(const NodalArgs& a, const Pend& q, 
 // neighbours.  Closes the proposal, or in precision 3 leaves it in shared
 // memory (the next entry of *pl, or *slot without a list) for
 // its float dS to be evaluated; returns whether it did.
-template <int G>
-constexpr int kGroupNbrs = G == 32 ? kHubDegree / 32 : kPairDegree / 16;
-
-template <class Ops, int G>
+template <int KN, class Ops, int G>
 __device__ __forceinline__ bool group_vertex(const NodalArgs& a, const Ops& ops, int v, uint32_t itr, int* tab,
                                              int* list, CtaTally* tl, const Grp<G>& g, unsigned long long* my_bytes,
                                              Pend* slot, PendList* pl) {
   using LD = typename Ops::Ld;
   using LDT = typename Ops::LdT;
-  constexpr int KN = kGroupNbrs<G>;
   int *key = tab, *two = tab + 8 * G, *twi = tab + 16 * G;
   const unsigned lanes_below = (1u << g.gl) - 1u;
   const VertexInfo vi = vertex_info<Ops>(a, v);
@@ -1064,18 +1060,18 @@ __device__ __forceinline__ bool group_vertex(const NodalArgs& a, const Ops& ops,
   }
 }
 
-// One warp per vertex of degree <= kHubDegree; 5 CTAs per SM so that a
-// batch of the bench workload (N/10 = 5000 vertices) runs in one wave.  The
-// float dS evaluates whole rows: the packing of coop_eval_sparse saves terms but
+// One warp per vertex of degree <= kBatchHubDegree; 4 CTAs per SM, so that a
+// lane's neighbours stay in registers (5 spilled: N = 20000, 113 ms a solve
+// against 101 ms).  The float dS evaluates whole rows: the packing of coop_eval_sparse saves terms but
 // adds latency to a warp that has a proposal of its own, and its queue takes
-// shared memory from the fifth CTA and the L1 (N = 20000, per-batch launches:
+// shared memory from the L1 (N = 20000, per-batch launches:
 // 141 ms a solve with it up to two edges a cell, 111 ms without; N = 50000: 251
 // and 221 ms; N = 3000 from one block per vertex: 245 and 235 ms).
 template <class Ops>
 __global__ void __launch_bounds__(kThreads, 4) k_nodal_propose(NodalArgs a, Ops ops) {
   __shared__ int s_tab[kWarps][3 * kHCap];
   // occupied slots other than r, s; then the float dS's terms
-  __shared__ __align__(16) int s_list[kWarps][kHubDegree];
+  __shared__ __align__(16) int s_list[kWarps][kBatchHubDegree];
   __shared__ Pend s_pend[Ops::kP == 3 ? kWarps : 1];
   __shared__ CtaTally s_tally;
   if (a.ctl->done) return;   // written by earlier launches only
@@ -1088,8 +1084,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_nodal_propose(NodalArgs a, Ops 
   unsigned long long my_bytes = 0;
   for (int v = a.beg + blockIdx.x * kWarps + wib; v < a.end; v += nwarps) {
     int* const tab = s_tab[wib];
-    const bool live = group_vertex(a, ops, v, itr, tab, s_list[wib], &s_tally, Grp<32>(lane), &my_bytes,
-                                   Ops::kP == 3 ? s_pend + wib : nullptr, nullptr);
+    const bool live = group_vertex<kBatchHubDegree / 32>(a, ops, v, itr, tab, s_list[wib], &s_tally, Grp<32>(lane),
+                                                         &my_bytes, Ops::kP == 3 ? s_pend + wib : nullptr, nullptr);
     if constexpr (Ops::kP == 3) {
       if (live) {   // warp-uniform
         const float f = ref32_eval(a, ops, s_pend[wib], tab, tab + kHCap, tab + 2 * kHCap,
@@ -1113,7 +1109,7 @@ struct HubShared {
   Pend pend;   // precision 3, without a list
 };
 
-// Proposal for one vertex of degree > kHubDegree by a whole CTA of NT
+// Proposal for one vertex of a larger degree by a whole CTA of NT
 // threads.  The last warp draws the target while the others fill the hash
 // of neighbour blocks (at most min(deg, B) entries: in `stab`, a shared
 // region of `scap` slots per array, or beyond that in the vertex's global
@@ -1324,7 +1320,7 @@ __device__ __forceinline__ void hub_vertex(const NodalArgs& a, const Ops& ops, i
   __syncthreads();
 }
 
-// one CTA per vertex of degree > kHubDegree, hash in dynamic shared memory
+// one CTA per vertex of degree > kBatchHubDegree, hash in dynamic shared memory
 // (`smem_cap` slots per array) or the vertex's global region
 template <class Ops>
 __global__ void __launch_bounds__(kHubThreads) k_nodal_propose_hub(NodalArgs a, Ops ops, const int32_t* hubs,
@@ -1845,7 +1841,7 @@ constexpr int kDeltaGlobalMinB = 256;     // from this B the phase kernel's appl
 // hub region stages the cooperative float dS
 constexpr int kSnapMaxB = 88;
 constexpr int kSnapSlots = 256;   // >= a hub table's capacity for B <= kSnapMaxB (2 * B rounded up to a power of 2)
-static_assert(kHubDegree >= 128, "the float dS's terms outgrow a warp's list");
+static_assert(kBatchHubDegree >= 128, "the float dS's terms outgrow a warp's list");
 static_assert(kMaxPend == 2 * kPWarps, "a wave's proposals outgrow the list");
 static_assert(3 * kSnapSlots + 2 * kSnapMaxB * kSnapMaxB + 3 * kSnapMaxB + 2 * kMaxPend * (4 * 16 + 4) <= 3 * kPHubSlots,
               "chunks of 16 blocks of a full list fit beside the tile copy");
@@ -2233,13 +2229,13 @@ __device__ __forceinline__ void unit_vertices(const NodalArgs& a, const Ops& ops
                                               CtaTally* tl, int lane, unsigned long long* my_bytes, PendList* pl) {
   int* list = wtab + 3 * kHCap;
   if (un.y == kUnitWarp) {
-    group_vertex(a, ops, un.x, itr, wtab, list, tl, Grp<32>(lane), my_bytes, nullptr, pl);
+    group_vertex<kHubDegree / 32>(a, ops, un.x, itr, wtab, list, tl, Grp<32>(lane), my_bytes, nullptr, pl);
   } else {
     const int h = lane >> 4;
     const int vv = h ? un.y : un.x;
     if (vv >= 0)
-      group_vertex(a, ops, vv, itr, wtab + h * (3 * kHCap / 2), list + h * kPairDegree, tl, Grp<16>(lane), my_bytes,
-                   nullptr, pl);
+      group_vertex<kPairDegree / 16>(a, ops, vv, itr, wtab + h * (3 * kHCap / 2), list + h * kPairDegree, tl,
+                                     Grp<16>(lane), my_bytes, nullptr, pl);
   }
   __syncwarp();
 }
