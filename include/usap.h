@@ -81,8 +81,7 @@ typedef struct usap_params {
   int32_t trace_kinds; /* trace events to emit: bit k-1 for kind k; 0 = all kinds */
   int32_t sweep_graphs;/* 1: record each stage's nodal sweep as a CUDA graph and replay it */
   int32_t persistent;  /* 1 (default): run each stage's nodal phase as one cooperative kernel
-                          when the tile is dense; 0: one launch per batch (the batched and
-                          served forms always use the cooperative kernel there). */
+                          when the tile is dense; 0: one launch per batch. */
   int32_t persistent_ctas; /* CTAs of the cooperative kernel (one per SM); 0 = every SM */
   int32_t precision;   /* 3 (default): the reference's float nodal dS, below.
                           0: every dS term in FP64, rounded to Q32 and summed exactly.
@@ -337,7 +336,8 @@ usap_status usap_op_nodal_batch_prec(usap_ctx* ctx, int32_t* part, int32_t B, in
  * out_assign must stay valid until the request is taken with poll or
  * wait.  A request's result is the same as usap_partition's for the same
  * graph and parameters.  As in the batched form, the requests' nodal phases
- * run side by side on shares of the SMs. */
+ * run side by side on shares of the SMs (with params.persistent = 0, as
+ * launches per batch that interleave with whatever else the GPU runs). */
 typedef struct usap_server usap_server;
 typedef struct usap_server_config {
   int32_t device;

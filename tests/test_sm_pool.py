@@ -73,3 +73,21 @@ def test_server_batch_and_contexts_at_once():
         t.join()
     srv.close()
     assert not bad, bad
+
+
+@pytest.mark.gpu
+def test_concurrent_forms_without_cooperative_launches():
+    """persistent = 0 holds in the batched and served forms too: launches per
+    batch, the same results."""
+    from usap_b200 import api, generator as gen, native as nat
+    graphs = [gen.generate(gen.SBMConfig(n=n, blocks=5, within=0.7, alpha=2.0, seed=n)) for n in (300, 900)]
+    alone = [api.partition(g.src, g.dst, None, g.n, params=nat.default_params(seed=1)) for g in graphs]
+    jobs, stats = api.batch_partition(graphs, [[1], [1]], nat.default_params(persistent=0))
+    assert stats["gang_launches"] == 0
+    srv = api.Server(0)
+    for g, (part, res), j in zip(graphs, alone, jobs):
+        p, r, _ = srv.wait(srv.submit(g.src, g.dst, None, g.n, params=nat.default_params(seed=1, persistent=0)))
+        assert np.array_equal(j["assign"], part) and j["result"]["S_q"] == res["S_q"]
+        assert np.array_equal(p, part) and r["S_q"] == res["S_q"]
+    srv.close()
+    assert api.batch_partition(graphs, [[1], [1]], nat.default_params())[1]["gang_launches"] > 0

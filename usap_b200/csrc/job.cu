@@ -1042,7 +1042,7 @@ void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res,
     const double model_d = model_S(n, hg_->e, B);
     trace_prev_moves_ = 0;
     const bool phase_ok = dense && !use_graphs && maxitr > 0 && B <= nodal_phase_max_blocks() && !trace_on(2);
-    const int pgrid = phase_ok && (p.persistent || concurrent_) ? nodal_phase_grid(device_) : 0;
+    const int pgrid = phase_ok && p.persistent ? nodal_phase_grid(device_) : 0;
     const int pmost = p.persistent_ctas > 0 ? std::min(pgrid, static_cast<int>(p.persistent_ctas)) : pgrid;
     if (pgrid > 0) {
       const PoolCtas ctas(*pool_, bs_, pmost, !concurrent_);
