@@ -193,10 +193,11 @@ void Job::free_vertex_state() {
 
 void Job::free_state() {
   free_vertex_state();
-  dfree(dout_); dfree(din_); dfree(batch_hub_); dfree(unit_ptr_); dfree(units_);
-  batch_hub_bs_ = 0;
-  batch_hub_cap_ = 0;
-  units_cap_ = 0;
+  dfree(dout_); dfree(din_);
+  for (Units& u : units_) {
+    dfree(u.batch_hub); dfree(u.unit_ptr); dfree(u.units);
+    u = Units{};
+  }
   dfree(M_); dfree(Mt_); dfree(CS_);
   dfree(Trow_); dfree(Tcol_);
   tcap_ = 0;
@@ -455,7 +456,7 @@ void Job::attach(std::shared_ptr<GraphResident> gr) {
     // replaced, and the caches built for the previous graph are dropped
     USAP_CUDA(cudaStreamSynchronize(st_));
     if (gr->hg.n > ncap_) free_vertex_state();
-    batch_hub_bs_ = 0;
+    for (Units& u : units_) u.bs = 0;
   }
   gr_ = std::move(gr);
   hg_ = &gr_->hg;
@@ -713,75 +714,93 @@ void Job::nodal_batch(int32_t* part, int32_t B, bool dense, int32_t beg, int32_t
   }
 }
 
+// a vertex per warp while a batch fits the grid's warps that way, else two
+bool Job::single_units(int grid) const { return bs_ <= static_cast<int64_t>(grid) * nodal_phase_warps(); }
+
+// The form that a phase needs follows from its CTAs, which may differ from stage
+// to stage beside other solves; what may be needed is built before CTAs are
+// taken from the pool, so that no SM waits for the host's pass and the copies.
+void Job::prepare_phase_units(int most) {
+  const bool single = single_units(most);
+  prepare_units(single);
+  if (single && !single_units(1) && (concurrent_ || pool_->shared())) prepare_units(false);
+}
+
+const Job::Units& Job::prepare_units(bool single) {
+  Units& u = units_[single ? 1 : 0];
+  if (u.bs == bs_) return u;
+  const int32_t n = hg_->n;
+  const int32_t nb = (n + bs_ - 1) / bs_;
+  const std::vector<int32_t>& hub_ids = gr_->hub_ids;
+  std::vector<int32_t> bh(static_cast<size_t>(nb) + 1);   // first hub of each batch
+  for (int32_t b = 0; b <= nb; b++) {
+    const int32_t v = static_cast<int32_t>(std::min<int64_t>(static_cast<int64_t>(b) * bs_, n));
+    bh[b] = static_cast<int32_t>(std::lower_bound(hub_ids.begin(), hub_ids.end(), v) - hub_ids.begin());
+  }
+  // work units: pairs of vertices of degree <= 64 (half-warps), single
+  // vertices of degree <= 192 (warps); hubs are proposed by whole CTAs
+  std::vector<int32_t> up(static_cast<size_t>(nb) + 1, 0);
+  std::vector<int32_t> un;
+  un.reserve(2 * static_cast<size_t>(n));
+  std::vector<int32_t> mid;
+  for (int32_t b = 0; b < nb; b++) {
+    const int32_t beg = b * bs_, end = std::min(n, beg + bs_);
+    int32_t pending = -1;
+    mid.clear();
+    for (int32_t v = beg; v < end; v++) {
+      const int64_t deg = (hg_->out_ptr[v + 1] - hg_->out_ptr[v]) + (hg_->in_ptr[v + 1] - hg_->in_ptr[v]);
+      if (deg > kHubDegree) continue;
+      if (single || deg > kPairDegree) {
+        mid.push_back(v);
+      } else if (pending < 0) {
+        pending = v;
+      } else {
+        un.push_back(pending);
+        un.push_back(v);
+        pending = -1;
+      }
+    }
+    if (pending >= 0) {
+      un.push_back(pending);
+      un.push_back(-1);
+    }
+    for (int32_t v : mid) {
+      un.push_back(v);
+      un.push_back(-2);
+    }
+    up[b + 1] = static_cast<int32_t>(un.size() / 2);
+  }
+  u.bs = 0;   // until everything is there
+  if (u.batch_cap < nb + 1) {
+    dfree(u.batch_hub);
+    dfree(u.unit_ptr);
+    u.batch_cap = 0;
+    dalloc(&u.batch_hub, nb + 1);
+    dalloc(&u.unit_ptr, nb + 1);
+    u.batch_cap = nb + 1;
+  }
+  if (u.cap < std::max<size_t>(un.size(), 2)) {
+    dfree(u.units);
+    u.cap = 0;
+    const size_t cap = std::max<size_t>(un.size(), 2);
+    int32_t* ua = nullptr;
+    dalloc(&ua, cap);
+    u.units = reinterpret_cast<int2*>(ua);
+    u.cap = cap;
+  }
+  USAP_CUDA(cudaMemcpyAsync(u.batch_hub, bh.data(), sizeof(int32_t) * bh.size(), cudaMemcpyHostToDevice, st_));
+  USAP_CUDA(cudaMemcpyAsync(u.unit_ptr, up.data(), sizeof(int32_t) * up.size(), cudaMemcpyHostToDevice, st_));
+  if (!un.empty())
+    USAP_CUDA(cudaMemcpyAsync(u.units, un.data(), sizeof(int32_t) * un.size(), cudaMemcpyHostToDevice, st_));
+  wait();
+  u.bs = bs_;
+  return u;
+}
+
 float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, int W, double thr,
                        double model_d, int32_t maxitr, int stats, int grid, bool timed) {
   const int32_t n = hg_->n;
-  const int32_t nb = (n + bs_ - 1) / bs_;
-  // a vertex per warp while a batch fits the grid's warps that way, else two
-  const bool single = bs_ <= static_cast<int64_t>(grid) * nodal_phase_warps();
-  if (batch_hub_bs_ != bs_ || units_single_ != single) {   // first hub of each batch, for this batch size
-    const std::vector<int32_t>& hub_ids = gr_->hub_ids;
-    std::vector<int32_t> bh(static_cast<size_t>(nb) + 1);
-    for (int32_t b = 0; b <= nb; b++) {
-      const int32_t v = static_cast<int32_t>(std::min<int64_t>(static_cast<int64_t>(b) * bs_, n));
-      bh[b] = static_cast<int32_t>(std::lower_bound(hub_ids.begin(), hub_ids.end(), v) - hub_ids.begin());
-    }
-    // work units: pairs of vertices of degree <= 64 (half-warps), single
-    // vertices of degree <= 192 (warps); hubs are proposed by whole CTAs
-    std::vector<int32_t> up(static_cast<size_t>(nb) + 1, 0);
-    std::vector<int32_t> un;
-    un.reserve(2 * static_cast<size_t>(n));
-    std::vector<int32_t> mid;
-    for (int32_t b = 0; b < nb; b++) {
-      const int32_t beg = b * bs_, end = std::min(n, beg + bs_);
-      int32_t pending = -1;
-      mid.clear();
-      for (int32_t v = beg; v < end; v++) {
-        const int64_t deg = (hg_->out_ptr[v + 1] - hg_->out_ptr[v]) + (hg_->in_ptr[v + 1] - hg_->in_ptr[v]);
-        if (deg > kHubDegree) continue;
-        if (single || deg > kPairDegree) {
-          mid.push_back(v);
-        } else if (pending < 0) {
-          pending = v;
-        } else {
-          un.push_back(pending);
-          un.push_back(v);
-          pending = -1;
-        }
-      }
-      if (pending >= 0) {
-        un.push_back(pending);
-        un.push_back(-1);
-      }
-      for (int32_t v : mid) {
-        un.push_back(v);
-        un.push_back(-2);
-      }
-      up[b + 1] = static_cast<int32_t>(un.size() / 2);
-    }
-    if (batch_hub_cap_ < nb + 1) {
-      dfree(batch_hub_);
-      dfree(unit_ptr_);
-      dalloc(&batch_hub_, nb + 1);
-      dalloc(&unit_ptr_, nb + 1);
-      batch_hub_cap_ = nb + 1;
-    }
-    if (units_cap_ < std::max<size_t>(un.size(), 2)) {
-      dfree(units_);
-      units_cap_ = std::max<size_t>(un.size(), 2);
-      int32_t* ua = nullptr;
-      dalloc(&ua, units_cap_);
-      units_ = reinterpret_cast<int2*>(ua);
-    }
-    int32_t* ud = reinterpret_cast<int32_t*>(units_);
-    USAP_CUDA(cudaMemcpyAsync(batch_hub_, bh.data(), sizeof(int32_t) * bh.size(), cudaMemcpyHostToDevice, st_));
-    USAP_CUDA(cudaMemcpyAsync(unit_ptr_, up.data(), sizeof(int32_t) * up.size(), cudaMemcpyHostToDevice, st_));
-    if (!un.empty())
-      USAP_CUDA(cudaMemcpyAsync(ud, un.data(), sizeof(int32_t) * un.size(), cudaMemcpyHostToDevice, st_));
-    wait();
-    batch_hub_bs_ = bs_;
-    units_single_ = single;
-  }
+  const Units& un = prepare_units(single_units(grid));
   PhaseArgs pa;
   pa.a = nodal_args(part, B, 0, 0, stage, seed, stats);
   pa.v = dense_view();
@@ -793,9 +812,9 @@ float Job::nodal_phase(int32_t* part, int32_t B, uint32_t stage, uint64_t seed, 
   pa.Mt = Mt_;
   pa.CS = CS_;
   pa.hubs = gr_->hubs_dev;
-  pa.batch_hub = batch_hub_;
-  pa.units = units_;
-  pa.unit_ptr = unit_ptr_;
+  pa.batch_hub = un.batch_hub;
+  pa.units = un.units;
+  pa.unit_ptr = un.unit_ptr;
   pa.chunk_ptr = g_.chunk_ptr;
   pa.n = n;
   pa.bs = bs_;
@@ -1045,6 +1064,7 @@ void Job::partition(const usap_params& p, int32_t* out_assign, usap_result* res,
     const int pgrid = phase_ok && p.persistent ? nodal_phase_grid(device_) : 0;
     const int pmost = p.persistent_ctas > 0 ? std::min(pgrid, static_cast<int>(p.persistent_ctas)) : pgrid;
     if (pgrid > 0) {
+      prepare_phase_units(pmost);
       const PoolCtas ctas(*pool_, bs_, pmost, !concurrent_);
       const auto tp0 = std::chrono::steady_clock::now();
       const float ms = nodal_phase(part, B, stage, seed, W, thr, model_d, maxitr, stats, ctas.n, stats != 0);

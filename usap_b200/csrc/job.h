@@ -304,7 +304,6 @@ class Job {
   int32_t bcap_ = 0, kcap_ = 0, dcap_ = 0, icap_ = 0;
   int32_t ncap_ = 0;          // vertices the per-vertex buffers hold
   int64_t hcap_ = 0;          // hub scratch slots
-  size_t units_cap_ = 0;      // ints of units_
   int32_t bs_ = 1;   // nodal batch size of the current solve
   int bar_test_hold_ = -1;                 // arm_barrier_test
   unsigned long long bar_test_timeout_ns_ = 0;
@@ -312,12 +311,19 @@ class Job {
   int32_t* move_to_ = nullptr;
   int32_t* from_ = nullptr;
   const int32_t* last_part_ = nullptr;   // slot holding the last solve's result
-  int32_t* batch_hub_ = nullptr;     // first hub of each batch of size bs_
-  int32_t* unit_ptr_ = nullptr;      // first work unit of each batch
-  int2* units_ = nullptr;            // work units of the persistent kernel
-  int32_t batch_hub_bs_ = 0;
-  bool units_single_ = false;        // units_ holds one vertex per unit
-  int32_t batch_hub_cap_ = 0;
+  // work units of the persistent kernel for batches of `bs` vertices (0: none
+  // yet): [0] with two vertices a warp, [1] with one
+  struct Units {
+    int32_t* batch_hub = nullptr;    // first hub of each batch
+    int32_t* unit_ptr = nullptr;     // first work unit of each batch
+    int2* units = nullptr;
+    int32_t bs = 0, batch_cap = 0;
+    size_t cap = 0;                  // ints of units
+  };
+  Units units_[2];
+  bool single_units(int grid) const;
+  void prepare_phase_units(int most);
+  const Units& prepare_units(bool single);
   int32_t *dout_ = nullptr, *din_ = nullptr;
   int *M_ = nullptr, *Mt_ = nullptr, *CS_ = nullptr;
   // precision mode 3: old-state term tables of the persistent kernel (ld_ x ld_ floats each)
