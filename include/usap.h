@@ -253,7 +253,7 @@ usap_status usap_ctx_test_barrier_timeout(usap_ctx* ctx, int32_t hold_cta, int64
 /* One job solves graphs[graph] with its own Philox seed (several jobs on the
  * same graph are independent chains).  Graphs are loaded once and shared.
  * Jobs run concurrently, each on its own stream driven by one of `workers`
- * host threads (0 = automatic; at most 8 solve at a time); their nodal phases
+ * host threads (0 = automatic; at most 8, more only load graphs); their nodal phases
  * run side by side, each as one cooperative launch on a share of the SMs that
  * follows its batch size, and their other work overlaps.  Every job's result
  * equals the result of solving it alone with the same seed. */
@@ -268,7 +268,7 @@ typedef struct usap_batch_job {
 typedef struct usap_batch_stats {
   double ms_total;      /* wall time of the whole call */
   double ms_load;       /* loading the graphs */
-  int32_t workers;
+  int32_t workers;      /* threads that solved */
   int64_t kernel_launches;
   int64_t gang_launches;  /* cooperative launches of the jobs' nodal phases */
   int64_t gang_phases;    /* nodal phases run in them (one each) */
@@ -328,8 +328,8 @@ usap_status usap_op_nodal_batch_prec(usap_ctx* ctx, int32_t* part, int32_t B, in
 /* --- served form: a partition service on one GPU --------------------------
  * The reference has no service; this replaces a caller running Graph_P
  * objects on its own threads.  usap_server_submit copies the edge list and
- * returns a ticket at once; worker threads take requests in arrival order
- * whenever a worker and a solver state are free (up to 8 solve at a time)
+ * returns a ticket at once; worker threads (at most 8, each with its own
+ * solver state) take requests in arrival order whenever a worker is free
  * and the request's device-memory footprint fits in what running requests
  * leave of the budget, so requests that arrive while others run start as
  * soon as a slot and memory free up and their kernels overlap on the GPU.
@@ -341,7 +341,7 @@ usap_status usap_op_nodal_batch_prec(usap_ctx* ctx, int32_t* part, int32_t B, in
 typedef struct usap_server usap_server;
 typedef struct usap_server_config {
   int32_t device;
-  int32_t workers;        /* worker threads (0: min(32, 2 x host threads)); at most 8 solve at a time */
+  int32_t workers;        /* worker threads, each solving a request at a time (0, or above 8: 8) */
   int64_t memory_budget;  /* bytes of device memory for admitted requests (0: 80% of free) */
   int32_t reserved[4];
 } usap_server_config;

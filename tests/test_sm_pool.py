@@ -91,3 +91,20 @@ def test_concurrent_forms_without_cooperative_launches():
         assert np.array_equal(p, part) and r["S_q"] == res["S_q"]
     srv.close()
     assert api.batch_partition(graphs, [[1], [1]], nat.default_params())[1]["gang_launches"] > 0
+
+
+@pytest.mark.gpu
+def test_workers_are_those_that_solve():
+    from usap_b200 import api, generator as gen, native as nat
+    g = gen.generate(gen.SBMConfig(n=200, blocks=4, within=0.8, alpha=5.0, seed=1))
+    for asked in (0, 3, 32):
+        srv = api.Server(0, workers=asked)
+        want = srv.stats()["workers"]
+        assert want == 3 if asked == 3 else 1 <= want <= 8
+        tickets = [srv.submit(g.src, g.dst, None, g.n) for _ in range(20)]
+        for t in tickets:
+            srv.wait(t)
+        assert 1 <= srv.stats()["peak_running"] <= want
+        srv.close()
+        _, stats = api.batch_partition([g], [list(range(12))], nat.default_params(), workers=asked)
+        assert stats["workers"] == (3 if asked == 3 else 8)

@@ -270,7 +270,7 @@ usap_status usap_ctx_test_barrier_timeout(usap_ctx* ctx, int32_t hold_cta, int64
   });
 }
 
-constexpr int kBatchWorkers = 64;
+constexpr int kBatchWorkers = 64;   // most threads that load a batch's graphs
 
 usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, const usap_params* p,
                                  usap_batch_job* jobs, int32_t njobs, int32_t workers,
@@ -284,8 +284,6 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
     usap_params_default(&def);
     const usap_params base = p ? *p : def;
     auto t0 = std::chrono::steady_clock::now();
-    int hw = static_cast<int>(std::thread::hardware_concurrency());
-    if (hw <= 0) hw = 8;
     USAP_CUDA(cudaSetDevice(device));
     int W = workers > 0 ? workers : kBatchWorkers;
     W = std::max(1, std::min(W, std::max(njobs, ngraphs)));
@@ -316,7 +314,7 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
     std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
       return res[jobs[a].graph]->hg.e > res[jobs[b].graph]->hg.e;
     });
-    // the first W solves (the largest graphs) would otherwise grow the memory
+    // the first solves (of the largest graphs) would otherwise grow the memory
     // pool while other solves' kernels run, which is slow: reserve it now
     {
       int64_t want = 0;
@@ -334,7 +332,8 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
     double phase_ms = 0.0;
     std::mutex phase_mu;
     std::vector<std::thread> th;
-    for (int w = 0; w < std::min(std::min(W, usap::kSolveSlots), std::max<int32_t>(njobs, 1)); w++)
+    const int solving = std::min(std::min(W, usap::kSolveSlots), std::max<int32_t>(njobs, 1));
+    for (int w = 0; w < solving; w++)
       th.emplace_back([&] {
         const auto lc0 = usap::launch_count();
         std::unique_ptr<usap::Job> job;
@@ -375,7 +374,7 @@ usap_status usap_batch_partition(const usap_graph* graphs, int32_t ngraphs, cons
     if (stats) {
       stats->ms_total = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
       stats->ms_load = std::chrono::duration<double, std::milli>(t1 - t0).count();
-      stats->workers = W;
+      stats->workers = solving;
       stats->kernel_launches = launches.load();
       stats->gang_launches = phases.load();
       stats->gang_phases = phases.load();

@@ -1,10 +1,10 @@
 // Served form: a partition service on one GPU.
 //
 // Requests arrive at any time (usap_server_submit copies the edge list and
-// returns a ticket at once).  A fixed set of worker threads, each owning a
-// solver state with its own CUDA streams, takes requests in arrival order
-// as soon as a worker is free and the request's device-memory footprint
-// fits in what the running requests leave of the budget; requests that
+// returns a ticket at once).  A fixed set of worker threads, with a solver
+// state and its CUDA streams for each, takes requests in arrival order as
+// soon as a worker is free and the request's device-memory footprint fits
+// in what the running requests leave of the budget; requests that
 // arrive while others run are admitted the moment a slot and memory free
 // up, and their kernels overlap those of the running requests on the
 // device.  Each request's graph, partition slots and block structures stay
@@ -77,10 +77,10 @@ class Server {
     budget_ = cfg.memory_budget > 0 ? cfg.memory_budget : static_cast<int64_t>(0.8 * static_cast<double>(free_b));
     int hw = static_cast<int>(std::thread::hardware_concurrency());
     if (hw <= 0) hw = 8;
-    const int nw = cfg.workers > 0 ? cfg.workers : std::min(32, 2 * hw);
+    const int nw = std::min(cfg.workers > 0 ? cfg.workers : 2 * hw, kSolveSlots);
     // the solver states are created up front, so that a missing or
     // unusable device fails here and not in a worker
-    for (int i = 0; i < std::min(nw, kSolveSlots); i++) {
+    for (int i = 0; i < nw; i++) {
       states_.push_back(std::make_unique<Job>(device_));
       states_.back()->set_concurrent(true);
       free_.push_back(states_.back().get());
@@ -181,17 +181,15 @@ class Server {
       Job* job = nullptr;
       {
         std::unique_lock<std::mutex> lk(mu_);
-        // arrival order; the oldest waiting request goes first as soon as a
-        // solver state is free and its footprint fits in the budget left by
-        // the running ones
+        // arrival order; the oldest waiting request goes first as soon as
+        // its footprint fits in the budget left by the running ones
         cv_work_.wait(lk, [&] {
-          return (stopping_ && queue_.empty()) ||
-                 (!queue_.empty() && !free_.empty() && admitted_ + queue_.front()->bytes <= budget_);
+          return (stopping_ && queue_.empty()) || (!queue_.empty() && admitted_ + queue_.front()->bytes <= budget_);
         });
         if (queue_.empty()) return;
         r = queue_.front();
         queue_.pop_front();
-        job = free_.back();
+        job = free_.back();   // the one used last: its buffers have grown
         free_.pop_back();
         admitted_ += r->bytes;
         running_++;
@@ -243,7 +241,7 @@ class Server {
   std::condition_variable cv_work_, cv_done_;
   std::deque<std::shared_ptr<Request>> queue_;
   std::unordered_map<int64_t, std::shared_ptr<Request>> requests_;
-  std::vector<std::unique_ptr<Job>> states_;   // shared by the workers
+  std::vector<std::unique_ptr<Job>> states_;   // as many as workers, free_ those not in use
   std::vector<Job*> free_;
   std::vector<std::thread> workers_;
   int64_t next_ticket_ = 1;
