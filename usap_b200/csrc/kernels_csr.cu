@@ -94,9 +94,8 @@ __global__ void k_scan_add(int32_t* __restrict__ out, int64_t n, const int32_t* 
 }
 
 // step 2: an edge into its bucket (arrival order), with its index
-__global__ void k_csr_scatter(const int32_t* __restrict__ key, const int32_t* __restrict__ val, int64_t e,
-                              const int32_t* __restrict__ ptr, int32_t* __restrict__ cursor,
-                              int32_t* __restrict__ tmp_eid) {
+__global__ void k_csr_scatter(const int32_t* __restrict__ key, int64_t e, const int32_t* __restrict__ ptr,
+                              int32_t* __restrict__ cursor, int32_t* __restrict__ tmp_eid) {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < e; i += stride) {
     const int32_t k = __ldg(key + i);
@@ -167,7 +166,7 @@ void csr_side(const int32_t* key, const int32_t* val, const int32_t* w, int64_t 
   k_csr_count<<<grid_for(e, kThreads), kThreads, 0, st>>>(key, w, e, cnt, deg);
   USAP_LAUNCHED();
   scan_exclusive_i32(cnt, m, ptr, st, alloc);
-  k_csr_scatter<<<grid_for(e, kThreads), kThreads, 0, st>>>(key, val, e, ptr, cursor, tmp);
+  k_csr_scatter<<<grid_for(e, kThreads), kThreads, 0, st>>>(key, e, ptr, cursor, tmp);
   USAP_LAUNCHED();
   k_csr_rank<<<static_cast<unsigned>((e + kThreads - 1) / kThreads), kThreads, 0, st>>>(ptr, key, e, tmp, val, w, idx, wo);
   USAP_LAUNCHED();

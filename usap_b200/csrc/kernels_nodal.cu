@@ -599,7 +599,11 @@ __device__ __noinline__ float ref32_nodal(const Ops ops, const int32_t* __restri
   // batch-start state), so that their L2 latency overlaps this round's
   // terms and chain.
   if (Trow) {
-    // the old-state terms from the batch's tables (written in this launch: L2 loads)
+    // the old-state terms from the batch's tables (written in this launch: L2
+    // loads).  Per-batch launches have none; the branch stays because the
+    // compiler's code for the rounds below is slower without it (N = 20000, 97 ms
+    // a solve with it, 112 ms without; a dozen other ways to write the rounds
+    // took 111 to 116 ms)
     const float* tr = Trow + static_cast<long long>(r) * tld;
     const float* ts = Trow + static_cast<long long>(s) * tld;
     const float* cr = Tcol + static_cast<long long>(r) * tld;
