@@ -311,7 +311,6 @@ int nodal_phase_grid(int device);
 // precision mode 3, persistent kernel: whether the float dS packs the non-zero
 // cells of its rows before it evaluates terms (a tile of B x B cells, `e` edges)
 bool float_ds_sparse(int64_t e, int32_t B);
-int64_t float_ds_table_max(int64_t e);   // most blocks of a tile that it does not pack, and so may have term tables
 int nodal_phase_warps();   // warps of one of its CTAs
 // largest B whose hub tables fit the persistent kernel's shared memory
 int nodal_phase_max_blocks();

@@ -40,7 +40,6 @@
 // moves) is otherwise read through L2 (ld.cg); the non-coherent path is
 // used only for data that no phase writes.  The phases
 // of concurrent solves run side by side, each on fewer CTAs.
-#include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <type_traits>
@@ -2589,10 +2588,6 @@ int nodal_phase_grid(int device) {
 // packed, 87 us whole; N = 50000 at B = 1526, 0.33: 385 against 294 us; N = 4999
 // at B = 625, 0.2: 26 against 33 us).
 bool float_ds_sparse(int64_t e, int32_t B) { return B > kSnapMaxB && 5 * e < static_cast<int64_t>(B) * B; }
-
-int64_t float_ds_table_max(int64_t e) {
-  return std::max<int64_t>(kSnapMaxB, static_cast<int64_t>(std::sqrt(5.0 * static_cast<double>(e))));
-}
 
 int nodal_phase_warps() { return kPWarps; }
 

@@ -13,6 +13,7 @@
 // seed.  Completion is read with usap_server_poll / usap_server_wait.
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <condition_variable>
 #include <cstring>
 #include <deque>
@@ -51,14 +52,14 @@ struct Request {
 // and e edges holds: the graph (edge list, both adjacency lists, edge
 // chunks, log table), the partition slots and per-vertex state, the sorted
 // views' sort buffers, the dense tile for B <= dense_max, and with the
-// float nodal dS its per-batch term tables (two floats per cell, up to
-// float_ds_table_max blocks).
+// float nodal dS its per-batch term tables (two floats per cell, B <= 4096).
 int64_t solve_footprint_bytes(int64_t n, int64_t e, int64_t dense_max, bool weighted, bool float_ds) {
   const int64_t d = std::min(n, std::max<int64_t>(dense_max, 1));
   const int64_t graph = (weighted ? 48 : 32) * e + 64 * n + 8 * (e + 1);
   const int64_t state = 72 * n + 160 * n + 112 * e;
   const int64_t tile = 8 * (d + 4) * (d + 4) + 4 * d * ((d + 127) / 128 + 1);
-  const int64_t dt = std::min(d, float_ds_table_max(e));
+  // (the float dS has term tables up to a fifth as many edges as cells)
+  const int64_t dt = std::min(d, std::max<int64_t>(4096, static_cast<int64_t>(std::sqrt(5.0 * static_cast<double>(e)))));
   const int64_t tables = float_ds ? 8 * (dt + 4) * (dt + 4) : 0;
   return graph + state + tile + tables + (8ll << 20);
 }
