@@ -52,13 +52,14 @@ struct Request {
 // and e edges holds: the graph (edge list, both adjacency lists, edge
 // chunks, log table), the partition slots and per-vertex state, the sorted
 // views' sort buffers, the dense tile for B <= dense_max, and with the
-// float nodal dS its per-batch term tables (two floats per cell, B <= 4096).
+// float nodal dS its per-batch term tables (two floats per cell).  The tables
+// are charged up to 4096 blocks; a solve has them up to the larger of 88
+// and sqrt(5 e) blocks, so most requests hold less.
 int64_t solve_footprint_bytes(int64_t n, int64_t e, int64_t dense_max, bool weighted, bool float_ds) {
   const int64_t d = std::min(n, std::max<int64_t>(dense_max, 1));
   const int64_t graph = (weighted ? 48 : 32) * e + 64 * n + 8 * (e + 1);
   const int64_t state = 72 * n + 160 * n + 112 * e;
   const int64_t tile = 8 * (d + 4) * (d + 4) + 4 * d * ((d + 127) / 128 + 1);
-  // (the float dS has term tables up to a fifth as many edges as cells)
   const int64_t dt = std::min(d, std::max<int64_t>(4096, static_cast<int64_t>(std::sqrt(5.0 * static_cast<double>(e)))));
   const int64_t tables = float_ds ? 8 * (dt + 4) * (dt + 4) : 0;
   return graph + state + tile + tables + (8ll << 20);
